@@ -119,6 +119,27 @@ def test_backward_kernels_agree_with_fp32(shape):
         _lib.check_status("attention")
 
 
+@pytest.mark.parametrize("shape", [(2, 706, 8, 8, 64), (2, 748, 16, 2, 64), (3, 161, 4, 2, 64), (2, 395, 8, 2, 128), (1, 1027, 8, 4, 128)])
+def test_backward_kernels_when_the_sequence_ends_inside_a_warp(shape):
+    """The last query tile holds a warp with rows on both sides of the end of the sequence; its off-diagonal tiles must
+    not split that warp around the warp-wide tensor-memory stores.  Tolerances as in the test above."""
+    from torchft_b200.ops import _lib
+    from torchft_b200.ops.attention import attention_bwd, attention_fwd
+
+    B, S, Hq, Hkv, D = shape
+    torch.manual_seed(5)
+    q, k, v = (torch.randn(B, S, h, D, device="cuda").to(torch.bfloat16) for h in (Hq, Hkv, Hkv))
+    do = torch.randn(B, S, Hq, D, device="cuda").to(torch.bfloat16)
+    o, lse = attention_fwd(q, k, v)
+    _, _, rq, rk, rv = reference(q, k, v, do)
+    for impl in ("smem", "tmem-dq", "split", "tmem"):
+        for _ in range(3):
+            dq, dk, dv = attention_bwd(do, q, k, v, o, lse, impl=impl)
+            for name, got, want in (("dq", dq, rq), ("dk", dk, rk), ("dv", dv, rv)):
+                assert rel(got, want) < 2e-2 and norm_rel(got, want) < 8e-3, (impl, name, rel(got, want), norm_rel(got, want))
+    _lib.check_status("attention")
+
+
 def test_attention_on_fused_qkv_views():
     from torchft_b200.ops.attention import attention_bwd, attention_fwd
 

@@ -168,6 +168,9 @@ attn_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       if (!mbar_wait(bar(SDP_FULL), t & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const bool diag = (it == jt);
+      // last key column this row keeps; the branch on it is one per warp (a sequence may end inside it)
+      const int last_key = row_ok ? (diag ? r : BLK - 1) : -1;
+      const bool masked = __any_sync(0xffffffffu, last_key < BLK - 1);
       float p[2][32], ds[2][32];
       // all four tensor-memory loads are issued before the single wait, so their latencies overlap
       uint32_t sv[2][32], dv[2][32];
@@ -180,10 +183,10 @@ attn_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
 #pragma unroll
       for (int cc = 0; cc < 2; ++cc) {
         const int c = half * 2 + cc;
-        if (diag || !row_ok) {
+        if (masked) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
-            const bool keep = row_ok && (c * 32 + i) <= r;
+            const bool keep = (c * 32 + i) <= last_key;
             p[cc][i] = keep ? fast_exp2(__uint_as_float(sv[cc][i]) * scale_log2 - lse) : 0.f;
             ds[cc][i] = p[cc][i] * (__uint_as_float(dv[cc][i]) - dl);
           }
@@ -386,6 +389,9 @@ attn_dkdv_split_kernel(const __grid_constant__ CUtensorMap tq, const __grid_cons
       if (!mbar_wait(bar(KS_S_FULL), t & 1, abort_flag)) { ok = false; break; }
       tc_fence_after();
       const bool diag = (it == jt);
+      // last key column this row keeps; the branch on it is one per warp (a sequence may end inside it)
+      const int last_key = row_ok ? (diag ? r : BLK - 1) : -1;
+      const bool masked = __any_sync(0xffffffffu, last_key < BLK - 1);
       float p[2][32];
       {
         uint32_t sv[2][32];
@@ -395,10 +401,10 @@ attn_dkdv_split_kernel(const __grid_constant__ CUtensorMap tq, const __grid_cons
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
           const int c = half * 2 + cc;
-          if (diag || !row_ok) {
+          if (masked) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
-              const bool keep = row_ok && (c * 32 + i) <= r;
+              const bool keep = (c * 32 + i) <= last_key;
               p[cc][i] = keep ? fast_exp2(__uint_as_float(sv[cc][i]) * scale_log2 - lse) : 0.f;
             }
           } else {  // mask-free fast path: every tile off the diagonal
@@ -609,10 +615,10 @@ attn_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
 #pragma unroll
       for (int cc = 0; cc < 2; ++cc) {
         const int c = half * 2 + cc;
-        if (diag || !row_ok) {
+        if (diag) {  // rows beyond the sequence need no mask: a row of dS reaches its own row of dQ only
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
-            const bool keep = row_ok && (c * 32 + i) <= r;
+            const bool keep = (c * 32 + i) <= r;
             const float p = keep ? fast_exp2(__uint_as_float(sv[cc][i]) * scale_log2 - lse) : 0.f;
             ds[cc][i] = p * (__uint_as_float(dv[cc][i]) - dl);
           }

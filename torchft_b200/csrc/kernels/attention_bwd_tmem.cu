@@ -190,10 +190,10 @@ attn_dq_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
       for (int cc = 0; cc < 2; ++cc) {
         const int c0 = half * 64 + cc * 32;
         float ds[32];
-        if (diag || !row_ok) {
+        if (diag) {  // rows beyond the sequence need no mask: a row of dS reaches its own row of dQ only
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
-            const bool keep = row_ok && (c0 + i) <= r;
+            const bool keep = (c0 + i) <= r;
             const float p = keep ? fast_exp2(__uint_as_float(sv[cc][i]) * scale_log2 - lse) : 0.f;
             ds[i] = p * (__uint_as_float(dv[cc][i]) - dl);
           }
