@@ -312,3 +312,53 @@ def test_diloco_fused_outer_step_matches_sgd():
             assert torch.equal(backup.views[i], p.detach())
             rp.data.copy_(p.detach().float())
             ref_outer.state[rp]["momentum_buffer"].copy_(outer.state[p]["momentum_buffer"])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("momentum,nesterov", [(0.9, True), (0.9, False), (0.0, False)])
+def test_outer_step_reads_and_writes_the_parameters_in_place(dtype, momentum, nesterov):
+    """Sizes around a vector and a block's chunk, a strided parameter, one at an odd address, more tensors than one table
+    holds.  The expected values follow the kernels' arithmetic (fp32, one rounding to ``dtype`` of the pseudo-gradient and
+    of the new weight), so a result may differ by one rounding of ``dtype`` where a multiply-add was contracted."""
+    from torchft_b200.local_sgd import _FlatBuckets
+    from torchft_b200.ops.outer_step import FusedOuterStep
+
+    chunk = 256 * 4 * (16 // torch.empty(0, dtype=dtype).element_size())
+    sizes = [1, 7, 8, 9, chunk - 1, chunk, chunk + 1, 3 * chunk + 5] + [3] * 125
+    base = torch.randn(sum(sizes) + 1, device=DEV).to(dtype)
+    params, at = [], 1  # from element 1 on: most of these views start at no 16-byte boundary
+    for n in sizes[:4]:
+        params.append(torch.nn.Parameter(base[at : at + n]))
+        at += n
+    params += [torch.nn.Parameter(torch.randn(n, device=DEV).to(dtype)) for n in sizes[4:]]
+    params.append(torch.nn.Parameter(torch.randn(48, 80, device=DEV).to(dtype).t()))
+    assert not params[-1].is_contiguous()
+    opt = torch.optim.SGD(params, lr=0.7, momentum=momentum, nesterov=nesterov)
+    backup, comm = _FlatBuckets(params, None, False), _FlatBuckets(params, None, False)
+    backup.copy_from_params()
+    fused = FusedOuterStep.maybe_create(params, backup, comm, opt)
+    old = [p.detach().clone() for p in params]
+    bufs = [None] * len(params)
+    ulp = 2.0**-7 if dtype == torch.bfloat16 else 2.0**-22
+    for _ in range(2):
+        with torch.no_grad():
+            for p in params:
+                p.add_((torch.randn(p.shape, device=DEV) * 0.05).to(dtype))
+        local = [p.detach().clone() for p in params]
+        fused.compute_pseudogradients()
+        for i, (p, q) in enumerate(zip(local, old)):
+            assert torch.equal(comm.views[i], (p.float() - q.float()).to(dtype))
+            assert torch.equal(params[i].detach(), p)
+        fused.apply_outer_update()
+        for i, p in enumerate(params):
+            g = comm.views[i].float() if p.is_contiguous() else (local[i].float() - old[i].float()).to(dtype).float()
+            bufs[i] = g if bufs[i] is None else momentum * bufs[i] + g
+            step = g if momentum == 0 else (g + momentum * bufs[i] if nesterov else bufs[i])
+            want = old[i].float() - 0.7 * step
+            assert ((p.detach().float() - want).abs() <= ulp * want.abs() + 1e-6).all()
+            assert torch.equal(backup.views[i], p.detach())
+            if momentum:
+                got = opt.state[p]["momentum_buffer"]
+                assert ((got - bufs[i]).abs() <= 2.0**-22 * (bufs[i].abs() + g.abs())).all()
+                bufs[i] = got.clone()
+            old[i] = p.detach().clone()

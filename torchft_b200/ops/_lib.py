@@ -36,8 +36,8 @@ _PROTOTYPES = {
     "tft_embedding_fwd": [P, P, P, L, I, P],
     "tft_embedding_bwd": [P, P, P, L, I, P],
     "tft_adamw": [P, P, P, P, L, F, F, F, F, F, I, F, P],
-    "tft_pseudograd": [P, P, L, I, P],
-    "tft_nesterov_outer": [P, P, P, L, F, F, I, I, I, P],
+    "tft_pseudograd": [P, P, P, I, P, P, I, P],
+    "tft_nesterov_outer": [P, P, P, I, P, P, P, F, F, I, I, I, P],
     "tft_attn_fwd": [P, P, P, P, P, I, I, I, I, I, I, I, I, F, P, P],
     "tft_attn_fwd_pair": [P, P, P, P, P, I, I, I, I, I, I, I, I, F, P, P],
     "tft_attn_bwd": [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, I, F, P, P],

@@ -4,7 +4,7 @@ Two kernels replace the reference's per-parameter ATen chain
 (``torchft/local_sgd.py:212-225``: sub, allreduce, divide, restore copy, SGD step, save
 copy):
 
-* ``pseudograd``: ``comm = local - global`` over the flat buckets in one pass;
+* ``pseudograd``: ``comm = local - global`` from the parameters into the flat buckets in one pass;
 * ``nesterov_update``: given the replica-averaged pseudo-gradient ``g``::
 
       buf    = momentum * buf + g
@@ -13,6 +13,8 @@ copy):
       param  = global;  backup = global
 
   reading g, global and buf once and writing param, backup and buf once.
+
+Both reach the parameters where they are; only the buckets are flat.
 
 With the NVLink process group the whole outer step is ONE kernel (``diloco_outer_kernel``):
 every replica averages its chunk of the local weights straight out of the peers' memory,
@@ -170,32 +172,56 @@ class FusedOuterStep:
             return None
         return cls(params, backup, comm, outer_optimizer)  # type: ignore[arg-type]
 
+    def _table(self, key: Tuple[torch.dtype, torch.device]):
+        """Addresses, bucket offsets and sizes of the parameters of one bucket, and the parameters that the kernels reach
+        only through their packed view (strided, or moved to another dtype or device since).  Built for every call:
+        nothing is kept by the address of a parameter."""
+        flat, (dtype, device) = self._comm.flat[key], key
+        idxs = self._comm.groups[key]
+        base, size = flat.data_ptr(), flat.element_size()
+        ptrs, offs, packed = [], [], []
+        for i in idxs:
+            p, view = self._params[i], self._comm.views[i]
+            assert view is not None
+            at = view.data_ptr()
+            offs.append((at - base) // size)
+            if p.is_contiguous() and p.dtype == dtype and p.device == device:
+                ptrs.append(p.data_ptr())
+            else:
+                ptrs.append(at)
+                packed.append(i)
+        n = len(idxs)
+        sizes = [self._params[i].numel() for i in idxs]
+        return (ctypes.c_void_p * n)(*ptrs), (ctypes.c_int64 * n)(*offs), (ctypes.c_int64 * n)(*sizes), n, packed
+
+    @staticmethod
+    def _launched(code: int, what: str) -> None:
+        _lib.check(max(-code, 0), what)
+        _lib.count_launch(code)
+
+    @torch.no_grad()
     def compute_pseudogradients(self) -> None:
-        """``comm = local - global`` (params are packed by the same kernel launch sequence)."""
-        self._comm.copy_from_params(non_blocking=True)
+        """``comm = local - global``, read straight from the live parameters."""
         lib = _lib.lib()
         for key, flat in self._comm.flat.items():
-            g = self._backup.flat[key]
-            code = lib.tft_pseudograd(
-                _lib.ptr(flat), _lib.ptr(g), ctypes.c_int64(flat.numel()),
-                ctypes.c_int(1 if flat.dtype == torch.bfloat16 else 0), _lib.stream_ptr(),
-            )
-            _lib.check(code, "tft_pseudograd")
-            _lib.count_launch()
+            ptrs, offs, sizes, n, packed = self._table(key)
+            for i in packed:
+                self._comm.views[i].copy_(self._params[i].data, non_blocking=True)  # type: ignore[union-attr]
+            code = lib.tft_pseudograd(ptrs, offs, sizes, n, _lib.ptr(flat), _lib.ptr(self._backup.flat[key]),
+                                      1 if flat.dtype == torch.bfloat16 else 0, _lib.stream_ptr())
+            self._launched(code, "tft_pseudograd")
 
+    @torch.no_grad()
     def apply_outer_update(self) -> None:
         g = self._opt.param_groups[0]
         lr, mu, nesterov = float(g["lr"]), float(g.get("momentum", 0.0)), bool(g.get("nesterov", False))
         lib = _lib.lib()
         for key, flat in self._comm.flat.items():
-            code = lib.tft_nesterov_outer(
-                _lib.ptr(flat), _lib.ptr(self._backup.flat[key]), _lib.ptr(self._momentum[key]),
-                ctypes.c_int64(flat.numel()), ctypes.c_float(lr), ctypes.c_float(mu),
-                ctypes.c_int(1 if nesterov else 0), ctypes.c_int(1 if self._first else 0),
-                ctypes.c_int(1 if flat.dtype == torch.bfloat16 else 0), _lib.stream_ptr(),
-            )
-            _lib.check(code, "tft_nesterov_outer")
-            _lib.count_launch()
+            ptrs, offs, sizes, n, packed = self._table(key)
+            code = lib.tft_nesterov_outer(ptrs, offs, sizes, n, _lib.ptr(flat), _lib.ptr(self._backup.flat[key]),
+                                          _lib.ptr(self._momentum[key]), lr, mu, 1 if nesterov else 0, 1 if self._first else 0,
+                                          1 if flat.dtype == torch.bfloat16 else 0, _lib.stream_ptr())
+            self._launched(code, "tft_nesterov_outer")
+            for i in packed:  # the kernel left their new values in the packed view
+                self._params[i].data.copy_(self._comm.views[i], non_blocking=True)  # type: ignore[arg-type]
         self._first = False
-        # comm now holds the new global weights; scatter them back into the parameters
-        self._comm.copy_to_params(non_blocking=True)
