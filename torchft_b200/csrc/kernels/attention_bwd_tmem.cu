@@ -16,14 +16,10 @@
 //                           dP^T = V dO_i^T put the KEY rows on the tensor-memory lanes, so P^T and
 //                           dS^T come out in the layout that dV += P^T dO_i and dK += dS^T Q_i need as
 //                           A operands.  The row statistics (log-sum-exp and delta) are then per
-//                           COLUMN; every item's 2 x 128 values are staged in shared memory.  Items
-//                           are cut into halves of 64 query columns that alternate between two sets
-//                           of score regions, so the softmax of one half runs under the MMAs of the
-//                           neighbouring ones.
+//                           COLUMN; every item's 2 x 128 values are staged in shared memory.
 //
-// A thread overwrites only tensor-memory columns it has read itself (each of the two threads of a row
-// packs its 64 values into the first 32 columns of its own 64-column half), so no thread can clobber
-// a value another warp still needs.  Waits are bounded as everywhere (common.cuh).
+// A thread overwrites only tensor-memory columns it has read itself, so no thread can clobber a value
+// another warp still needs.  Waits are bounded as everywhere (common.cuh).
 #include "attention_common.cuh"
 
 namespace tft {
@@ -255,28 +251,55 @@ int launch_dq_tmem(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorM
 }
 
 // ------------------------------------------------------------------ dK, dV (transposed scores)
-// An item (one query head of the group x one query tile) is processed as two HALF ITEMS of 64 query
-// columns.  Each half item has its own pair of 64-column score regions, so while the softmax threads
-// work on one half item the tensor cores run the gradient products of the previous one and the score
-// products of the next: the ping-pong that a full item, which would fill the score regions alone,
-// cannot have next to two 128-column accumulators.
+// An item is one query head of the group x one query tile.  Tensor-core order per item t:
+//
+//   dV(t) queries 0-63 | dV(t) 64-127 | S(t + LA) | dK(t) 0-63 | dK(t) 64-127 | dP(t + 1)
+//
+// The softmax threads work on the first 64 query columns of an item before the last 64 and announce the two halves
+// separately, so the gradient products start under the second half of the exponentials.  S(t + LA) follows dV(t)
+// directly and runs under the formation of dS(t); dP(t + 1) comes last, where nobody waits for it.  Head dimension 64
+// leaves room for two score regions (LA = 2): the scores of the next item are then ready before they are asked for.
+// With head dimension 128 the two accumulators take half of the tensor memory and LA is 1.
+// What bounds it: the exponentials of an item take 1024 cycles of the MUFU unit (16 a cycle and SM) and the softmax threads
+// about as long again for loads, dS, packing and stores; the four products take 2048 cycles at head dimension 128 and
+// 1024 at 64.  Measured against attn_dkdv_split_kernel (P and dS through shared memory): 233 us for 275 (one sequence of
+// 4096, 32/8 heads of 128), 104 for 129 (two of 2048, 32/8 heads of 64).  At head dimension 128 the tensor pipe is issued
+// to without a break (80 to 108 cycles an instruction, 64 nominal: the operands of S and dP come from shared memory at
+// its full rate); at 64 the softmax threads set the pace.
 template <int HD>
 struct DkvTmemSmem {
+  static constexpr int LA = HD == 64 ? 2 : 1;  // score regions: how many items ahead S is issued
+  static constexpr int QST = LA + 1;           // Q(t) is read by dK(t) after S(t + LA) has been issued
+  static constexpr int DST = 2;
   static constexpr uint32_t TILE = BLK * HD * 2;
-  static constexpr uint32_t K = 0, V = TILE, Q = 2 * TILE /*2 stages*/, DO = 4 * TILE /*2 stages*/;
-  static constexpr uint32_t STATS = 6 * TILE;  // float [2 buffers][lse 128 | delta 128]
+  static constexpr uint32_t K = 0, V = TILE, Q = 2 * TILE, DO = Q + QST * TILE;
+  static constexpr uint32_t STATS = DO + DST * TILE;  // float [2 buffers][lse 128 | delta 128]
   static constexpr uint32_t BARS = STATS + 2 * 2 * BLK * 4;
   static constexpr uint32_t TOTAL = BARS + 256 + 1024;
 };
 enum DkvTmemBar {
-  TK_KV_FULL = 0, TK_Q_FULL0, TK_Q_FULL1, TK_DO_FULL0, TK_DO_FULL1, TK_Q_EMPTY0, TK_Q_EMPTY1, TK_DO_EMPTY0, TK_DO_EMPTY1,
-  TK_SDP_FULL0, TK_SDP_FULL1, TK_PDS_READY0, TK_PDS_READY1, TK_ACC_DONE, NUM_TK_BARS
+  TK_KV_FULL = 0, TK_Q_FULL0, TK_Q_EMPTY0 = TK_Q_FULL0 + 3, TK_DO_FULL0 = TK_Q_EMPTY0 + 3, TK_DO_EMPTY0 = TK_DO_FULL0 + 2,
+  TK_S_FULL0 = TK_DO_EMPTY0 + 2, TK_DP_FULL = TK_S_FULL0 + 2, TK_P_LO, TK_P_HI, TK_DS_LO, TK_DS_HI, TK_ACC_DONE, NUM_TK_BARS
 };
 
-// Column of k-step kk (16 of a half item's 64 query columns) inside a 64-column region whose two
-// threads per row each packed their 32 values into the first 16 columns of their own 32-column half.
-__device__ __forceinline__ uint32_t half_item_kstep(uint32_t region, int kk) {
-  return region + (kk < 2 ? kk * 8 : 32 + (kk - 2) * 8);
+// Column of k-step kk (16 of an item's 128 query columns) inside a 128-column region.  The thread of half h of a key row
+// owns columns [32 h, 32 h + 32) and [64 + 32 h, 64 + 32 h + 32) and packs each 32 values into the first 16 of their columns.
+__device__ __forceinline__ uint32_t dkv_kstep(uint32_t region, int kk) { return region + (kk >> 1) * 32 + (kk & 1) * 8; }
+
+// Barrier over the 256 softmax threads that tells all of them whether any passed `mine`.
+__device__ __forceinline__ bool softmax_threads_any(bool mine) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.or.pred.aligned q, 1, 256, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t"
+      "}\n"
+      : "=r"(any)
+      : "r"(mine ? 1u : 0u)
+      : "memory");
+  return any != 0;
 }
 
 template <int HD>
@@ -287,6 +310,7 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
                       __nv_bfloat16* __restrict__ dV, int S, int Hq, int Hkv, long long lddk, long long lddv, float scale,
                       float scale_log2, int* status) {
   using L = DkvTmemSmem<HD>;
+  constexpr int LA = L::LA, QST = L::QST, DST = L::DST;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -302,12 +326,10 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
   const int jt = blockIdx.x / Hkv;  // key tile; early key tiles have the most work and come first
   const int kv_head = blockIdx.x % Hkv, batch = blockIdx.y;
   const int G = Hq / Hkv;
-  const int per_head = n_tiles - jt;
-  const int n_items = G * per_head;  // (query head of the group, query tile at or after the key tile)
-  const int n_halves = 2 * n_items;
+  const int n_items = G * (n_tiles - jt);  // (query head of the group, query tile at or after the key tile)
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < NUM_TK_BARS; ++i) mbar_init(bar(i), (i == TK_PDS_READY0 || i == TK_PDS_READY1) ? 256 : 1);
+    for (int i = 0; i < NUM_TK_BARS; ++i) mbar_init(bar(i), (i >= TK_P_LO && i <= TK_DS_HI) ? 8 : 1);  // one arrival per softmax warp
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tq);
@@ -323,136 +345,178 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  // region set x of half item hh (x = hh & 1): S^T (later P^T) at x * 128, dP^T (later dS^T) at x * 128 + 64;
-  // key rows on the lanes everywhere
-  auto t_st = [&](int hh) { return tmem_base + static_cast<uint32_t>(hh & 1) * 128u; };
-  auto t_dpt = [&](int hh) { return tmem_base + static_cast<uint32_t>(hh & 1) * 128u + 64u; };
-  const uint32_t t_dv = tmem_base + 256, t_dk = tmem_base + 256 + HD;
+  // key rows on the lanes everywhere: S^T (later P^T) of item t, dP^T (later dS^T), the two accumulators
+  auto t_st = [&](int t) { return tmem_base + (LA == 2 ? static_cast<uint32_t>(t & 1) * 128u : 0u); };
+  const uint32_t t_dpt = tmem_base + LA * 128u, t_dv = t_dpt + 128u, t_dk = t_dv + HD;
 
   if (warp == 0) {
     if (lane == 0) {
       mbar_expect_tx(bar(TK_KV_FULL), 2 * L::TILE);
       load_tile<HD>(base + L::K, &tk, bar(TK_KV_FULL), kv_head, jt * BLK, batch);
       load_tile<HD>(base + L::V, &tv, bar(TK_KV_FULL), kv_head, jt * BLK, batch);
+      int it = jt, head = kv_head * G;
       for (int t = 0; t < n_items; ++t) {
-        const int head = kv_head * G + t / per_head;
-        const int it = jt + t % per_head;
-        const int st = t & 1;
-        const uint32_t free_parity = ((t >> 1) & 1) ^ 1;
-        if (!mbar_wait(bar(TK_Q_EMPTY0 + st), free_parity, abort_flag)) break;
-        mbar_expect_tx(bar(TK_Q_FULL0 + st), L::TILE);
-        load_tile<HD>(base + L::Q + st * L::TILE, &tq, bar(TK_Q_FULL0 + st), head, it * BLK, batch);
-        if (!mbar_wait(bar(TK_DO_EMPTY0 + st), free_parity, abort_flag)) break;
-        mbar_expect_tx(bar(TK_DO_FULL0 + st), L::TILE);
-        load_tile<HD>(base + L::DO + st * L::TILE, &tdo, bar(TK_DO_FULL0 + st), head, it * BLK, batch);
+        const int qs = t % QST, ds = t % DST;
+        if (!mbar_wait(bar(TK_Q_EMPTY0 + qs), ((t / QST) & 1) ^ 1, abort_flag)) break;
+        mbar_expect_tx(bar(TK_Q_FULL0 + qs), L::TILE);
+        load_tile<HD>(base + L::Q + qs * L::TILE, &tq, bar(TK_Q_FULL0 + qs), head, it * BLK, batch);
+        if (!mbar_wait(bar(TK_DO_EMPTY0 + ds), ((t / DST) & 1) ^ 1, abort_flag)) break;
+        mbar_expect_tx(bar(TK_DO_FULL0 + ds), L::TILE);
+        load_tile<HD>(base + L::DO + ds * L::TILE, &tdo, bar(TK_DO_FULL0 + ds), head, it * BLK, batch);
+        if (++it == n_tiles) {
+          it = jt;
+          ++head;
+        }
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      constexpr uint32_t idesc_s = make_idesc_bf16(BLK, 64, false, false);   // 128 keys x 64 queries
+      constexpr uint32_t idesc_s = make_idesc_bf16(BLK, BLK, false, false);  // 128 keys x 128 queries
       constexpr uint32_t idesc_g = make_idesc_bf16(BLK, HD, false, true);
-      // S^T = K Q^T and dP^T = V dO^T for the 64 query rows of half item hh: the key tile is the A
-      // operand (keys land on the lanes); the B operand is rows [64 s, 64 s + 64) of the item's Q / dO tile
-      auto issue_sdp = [&](int hh) -> bool {
-        const int t = hh >> 1, s = hh & 1, st = t & 1;
-        if (s == 0) {  // first half of an item: its Q / dO stage must have landed
-          const uint32_t ph = (t >> 1) & 1;
-          if (!mbar_wait(bar(TK_Q_FULL0 + st), ph, abort_flag) || !mbar_wait(bar(TK_DO_FULL0 + st), ph, abort_flag)) return false;
-          tc_fence_after();
-        }
-        const uint32_t sq = base + L::Q + st * L::TILE + s * 8192, sdo = base + L::DO + st * L::TILE + s * 8192;
+      // S^T = K Q^T of item t: the key tile is the A operand, so keys land on the lanes
+      auto issue_s = [&](int t) -> bool {
+        const int qs = t % QST;
+        if (!mbar_wait(bar(TK_Q_FULL0 + qs), (t / QST) & 1, abort_flag)) return false;
+        tc_fence_after();
+        const uint32_t sq = base + L::Q + qs * L::TILE;
 #pragma unroll
-        for (int k = 0; k < HD / 16; ++k) umma_bf16(t_st(hh), kmajor_desc(base + L::K, k), kmajor_desc(sq, k), idesc_s, k != 0);
-#pragma unroll
-        for (int k = 0; k < HD / 16; ++k) umma_bf16(t_dpt(hh), kmajor_desc(base + L::V, k), kmajor_desc(sdo, k), idesc_s, k != 0);
-        umma_commit(bar(TK_SDP_FULL0 + (hh & 1)));
+        for (int k = 0; k < HD / 16; ++k) umma_bf16(t_st(t), kmajor_desc(base + L::K, k), kmajor_desc(sq, k), idesc_s, k != 0);
+        umma_commit(bar(TK_S_FULL0 + t % LA));
         return true;
       };
-      bool ok = mbar_wait(bar(TK_KV_FULL), 0, abort_flag);
-      if (ok && n_halves > 0) ok = issue_sdp(0) && issue_sdp(1);
-      for (int hh = 0; hh < n_halves && ok; ++hh) {
-        const int t = hh >> 1, s = hh & 1, st = t & 1;
-        const uint32_t sq = base + L::Q + st * L::TILE, sdo = base + L::DO + st * L::TILE;
-        if (!mbar_wait(bar(TK_PDS_READY0 + (hh & 1)), (hh >> 1) & 1, abort_flag)) { ok = false; break; }
+      auto issue_dp = [&](int t) -> bool {  // dP^T = V dO^T of item t
+        const int ds = t % DST;
+        if (!mbar_wait(bar(TK_DO_FULL0 + ds), (t / DST) & 1, abort_flag)) return false;
         tc_fence_after();
-        // dV += P^T dO and dK += dS^T Q over this half item's 64 query rows: A from tensor memory
+        const uint32_t sdo = base + L::DO + ds * L::TILE;
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          umma_bf16_ts(t_dv, half_item_kstep(t_st(hh), kk), mnmajor_desc(sdo, 4 * s + kk), idesc_g, (hh | kk) != 0);
-        if (s == 1) umma_commit(bar(TK_DO_EMPTY0 + st));
+        for (int k = 0; k < HD / 16; ++k) umma_bf16(t_dpt, kmajor_desc(base + L::V, k), kmajor_desc(sdo, k), idesc_s, k != 0);
+        umma_commit(bar(TK_DP_FULL));
+        return true;
+      };
+      // acc (+)= A B over the item's query rows [64 half, 64 half + 64): A = P^T or dS^T from tensor memory
+      auto issue_grad = [&](uint32_t acc, uint32_t a_region, uint32_t b_tile, int t, int half) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          umma_bf16_ts(t_dk, half_item_kstep(t_dpt(hh), kk), mnmajor_desc(sq, 4 * s + kk), idesc_g, (hh | kk) != 0);
-        if (s == 1) umma_commit(bar(TK_Q_EMPTY0 + st));
-        // in order behind them: the scores of half item hh + 2 go into the regions just consumed
-        if (hh + 2 < n_halves && !issue_sdp(hh + 2)) { ok = false; break; }
+        for (int kk = 0; kk < 4; ++kk) {
+          const int k = half * 4 + kk;
+          umma_bf16_ts(acc, dkv_kstep(a_region, k), mnmajor_desc(b_tile, k), idesc_g, (t | k) != 0);
+        }
+      };
+      bool ok = mbar_wait(bar(TK_KV_FULL), 0, abort_flag);
+      if (ok && n_items > 0) ok = issue_s(0) && issue_dp(0);
+      if (ok && LA == 2 && n_items > 1) ok = issue_s(1);
+      for (int t = 0; t < n_items && ok; ++t) {
+        const int qs = t % QST, ds = t % DST;
+        const uint32_t sq = base + L::Q + qs * L::TILE, sdo = base + L::DO + ds * L::TILE;
+        if (!mbar_wait(bar(TK_P_LO), t & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        issue_grad(t_dv, t_st(t), sdo, t, 0);
+        if (!mbar_wait(bar(TK_P_HI), t & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        issue_grad(t_dv, t_st(t), sdo, t, 1);
+        umma_commit(bar(TK_DO_EMPTY0 + ds));
+        // in order behind dV(t), which was the last reader of the region
+        if (t + LA < n_items && !issue_s(t + LA)) { ok = false; break; }
+        if (!mbar_wait(bar(TK_DS_LO), t & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        issue_grad(t_dk, t_dpt, sq, t, 0);
+        if (!mbar_wait(bar(TK_DS_HI), t & 1, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        issue_grad(t_dk, t_dpt, sq, t, 1);
+        umma_commit(bar(TK_Q_EMPTY0 + qs));
+        if (t + 1 < n_items && !issue_dp(t + 1)) { ok = false; break; }
       }
       if (ok) umma_commit(bar(TK_ACC_DONE));
     }
   } else {
     const int q = warp & 3;
-    const int hf = (warp - 2) >> 2;    // two threads per key row: columns [0,32) and [32,64) of the half item
-    const int r = q * 32 + lane;       // key row inside the tile
+    const int hf = (warp - 2) >> 2;  // two threads per key row, each with 32 of the first and 32 of the last 64 query columns
+    const int r = q * 32 + lane;     // key row inside the tile
     const int e = (warp - 2) * 32 + lane;  // 0..255: which statistic this thread fetches per item
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     bool ok = true;
-    // statistic of item t for this thread's slot: log-sum-exp (slots 0..127) or delta (128..255) of one
+    // statistic of a query tile for this thread's slot: log-sum-exp (slots 0..127) or delta (128..255) of one
     // query row; +inf as log-sum-exp of a row beyond the sequence turns its probabilities into zeros
-    auto fetch_stat = [&](int t) -> float {
-      const int head = kv_head * G + t / per_head;
-      const int qrow = (jt + t % per_head) * BLK + (e & 127);
+    auto fetch_stat = [&](int head, int it) -> float {
+      const int qrow = it * BLK + (e & 127);
       const long long at = (static_cast<long long>(batch) * Hq + head) * S + qrow;
       if (e < 128) return qrow < S ? LSE[at] : INFINITY;
       return qrow < S ? delta[at] : 0.f;
     };
-    float next_stat = n_items > 0 ? fetch_stat(0) : 0.f;
-    for (int hh = 0; hh < n_halves; ++hh) {
-      const int t = hh >> 1, s = hh & 1;
-      const int it = jt + t % per_head;
+    int it = jt, head = kv_head * G;
+    float next_stat = n_items > 0 ? fetch_stat(head, it) : 0.f;
+    for (int t = 0; t < n_items; ++t) {
+      const bool diag = it == jt;
+      const int q_end = S - it * BLK;                  // query columns at or beyond this one do not exist
+      const bool masked = diag || q_end < BLK;         // the same for the whole block
       float* my_stats = stats + (t & 1) * 2 * BLK;
-      if (s == 0) {
-        my_stats[e] = next_stat;
-        if (t + 1 < n_items) next_stat = fetch_stat(t + 1);  // travels while this item is processed
+      my_stats[e] = next_stat;
+      if (++it == n_tiles) {
+        it = jt;
+        ++head;
       }
-      const bool got = mbar_wait(bar(TK_SDP_FULL0 + (hh & 1)), (hh >> 1) & 1, abort_flag);
-      if (s == 0) {
-        asm volatile("bar.sync 1, 256;" ::: "memory");  // every statistic of this item is in shared memory
-        if (*abort_flag) { ok = false; break; }  // uniform: whoever gave up set the flag before the barrier
-      } else if (!__all_sync(0xffffffffu, got)) {
-        ok = false;
-        break;
-      }
+      if (t + 1 < n_items) next_stat = fetch_stat(head, it);  // travels while this item is processed
+      ok = __all_sync(0xffffffffu, mbar_wait(bar(TK_S_FULL0 + t % LA), (t / LA) & 1, abort_flag)) && ok;
+      // every statistic of this item is in shared memory; all 256 threads leave together if one of them gave up
+      ok = !softmax_threads_any(!ok);
+      if (!ok) break;
       tc_fence_after();
-      const bool diag = (it == jt);
-      const int c0 = s * 64 + hf * 32;  // first query column (inside the tile) of this thread's 32
-      const uint32_t my_st = t_st(hh) + lane_addr + hf * 32, my_dpt = t_dpt(hh) + lane_addr + hf * 32;
-      uint32_t sv[32], dv[32];
-      tmem_ld_32x32(my_st, sv);
-      tmem_ld_32x32(my_dpt, dv);
-      tmem_ld_wait();
-      float p[32], ds[32];
+      float p[2][32];
+      {
+        uint32_t sv[2][32];
 #pragma unroll
-      for (int i4 = 0; i4 < 8; ++i4) {
-        const float4 ls = *reinterpret_cast<const float4*>(my_stats + c0 + i4 * 4);
-        const float4 dl = *reinterpret_cast<const float4*>(my_stats + BLK + c0 + i4 * 4);
-        const float lsv[4] = {ls.x, ls.y, ls.z, ls.w}, dlv[4] = {dl.x, dl.y, dl.z, dl.w};
+        for (int h = 0; h < 2; ++h) tmem_ld_32x32(t_st(t) + lane_addr + h * 64 + hf * 32, sv[h]);
+        tmem_ld_wait();
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int i = i4 * 4 + u;
-          float pv = fast_exp2(__uint_as_float(sv[i]) * scale_log2 - lsv[u]);
-          if (diag && (c0 + i) < r) pv = 0.f;  // causal: query column >= key row
-          p[i] = pv;
-          ds[i] = pv * (__uint_as_float(dv[i]) - dlv[u]);
+        for (int h = 0; h < 2; ++h) {
+          const int c0 = h * 64 + hf * 32;
+#pragma unroll
+          for (int i4 = 0; i4 < 8; ++i4) {
+            const float4 ls = *reinterpret_cast<const float4*>(my_stats + c0 + i4 * 4);
+            const float lsv[4] = {ls.x, ls.y, ls.z, ls.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) p[h][i4 * 4 + u] = fast_exp2(__uint_as_float(sv[h][i4 * 4 + u]) * scale_log2 - lsv[u]);
+          }
+          if (masked) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i)  // causal: query column >= key row
+              if ((diag && c0 + i < r) || c0 + i >= q_end) p[h][i] = 0.f;
+          }
+          uint32_t packed[16];
+          pack32(p[h], packed);
+          tmem_st_32x16(t_st(t) + lane_addr + c0, packed);  // over score columns this thread has already read
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();  // the lanes' stores are ordered before the one arrival of the warp
+          if (lane == 0) mbar_arrive(bar(h == 0 ? TK_P_LO : TK_P_HI));
         }
       }
-      uint32_t packed[16];
-      pack32(p, packed);
-      tmem_st_32x16(my_st, packed);   // over score columns this thread has already read
-      pack32(ds, packed);
-      tmem_st_32x16(my_dpt, packed);
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(bar(TK_PDS_READY0 + (hh & 1)));
+      ok = __all_sync(0xffffffffu, mbar_wait(bar(TK_DP_FULL), t & 1, abort_flag));  // acted upon at the next item's barrier
+      tc_fence_after();
+      {
+        uint32_t dv[2][32];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) tmem_ld_32x32(t_dpt + lane_addr + h * 64 + hf * 32, dv[h]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int c0 = h * 64 + hf * 32;
+#pragma unroll
+          for (int i4 = 0; i4 < 8; ++i4) {
+            const float4 dl = *reinterpret_cast<const float4*>(my_stats + BLK + c0 + i4 * 4);
+            const float dlv[4] = {dl.x, dl.y, dl.z, dl.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) p[h][i4 * 4 + u] *= __uint_as_float(dv[h][i4 * 4 + u]) - dlv[u];
+          }
+          uint32_t packed[16];
+          pack32(p[h], packed);
+          tmem_st_32x16(t_dpt + lane_addr + c0, packed);
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(h == 0 ? TK_DS_LO : TK_DS_HI));
+        }
+      }
     }
     if (ok && n_items > 0) {
       const bool done = mbar_wait(bar(TK_ACC_DONE), 0, abort_flag);

@@ -1,5 +1,5 @@
 """Causal grouped-query flash attention on tcgen05 tensor cores
-(``csrc/kernels/attention_fwd_pair.cu``, ``attention_fwd.cu`` and ``attention_bwd.cu``).
+(``csrc/kernels/attention_fwd_pair.cu``, ``attention_fwd.cu``, ``attention_bwd_tmem.cu`` and ``attention_bwd.cu``).
 
 Two forward kernels with one contract: ``pair`` runs two query tiles per CTA in ping-pong, keeps P in
 tensor memory and accumulates the output there; ``single`` runs one tile per CTA with P through shared
@@ -46,7 +46,7 @@ def attention_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: Opti
     return o, lse
 
 
-BWD_IMPL = os.environ.get("TFT_ATTN_BWD", "split")
+BWD_IMPL = os.environ.get("TFT_ATTN_BWD", "tmem")
 assert BWD_IMPL in ("smem", "tmem", "tmem-dq", "split"), f"TFT_ATTN_BWD must be 'smem', 'tmem', 'tmem-dq' or 'split', not {BWD_IMPL!r}"
 
 
@@ -56,7 +56,7 @@ def attention_bwd(do: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.T
                   impl: Optional[str] = None) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     """Gradients ``(dq, dk, dv)``; ``out`` may name preallocated (possibly strided) destinations.
 
-    ``impl="smem"``: P and dS go through shared memory (``attention_bwd.cu``); ``"tmem"``: they stay in
+    ``impl="smem"``: P and dS go through shared memory (``attention_bwd.cu``); ``"tmem"`` (the default): they stay in
     tensor memory as MMA operands (``attention_bwd_tmem.cu``); ``"tmem-dq"``: the dQ kernel of the latter behind
     the dK/dV kernel of the former; ``"split"``: the same with the dK/dV kernel whose S and dP products run as
     separate pipelines.  Default from ``TFT_ATTN_BWD``."""
