@@ -68,7 +68,7 @@ attn_dq_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
   volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(smem + L::BARS + 8 * NUM_TQ_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::BARS + 8 * NUM_TQ_BARS + 8);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   const int n_tiles = (S + BLK - 1) / BLK;
   const int qt = n_tiles - 1 - blockIdx.x / Hq;  // heaviest first over all heads
   const int head = blockIdx.x % Hq, batch = blockIdx.y;
@@ -111,50 +111,51 @@ attn_dq_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const uint32_t leader = elect_one();
       constexpr uint32_t idesc_s = make_idesc_bf16(BLK, BLK, false, false);
       constexpr uint32_t idesc_q = make_idesc_bf16(BLK, HD, false, true);
       auto issue_s = [&](int j) -> bool {  // S(j) = Q K_j^T into the score region of tile j
         const int ks = j % KS;
-        if (!mbar_wait(bar(TQ_K_FULL0 + ks), (j / KS) & 1, abort_flag)) return false;
+        if (!mbar_wait_warp(bar(TQ_K_FULL0 + ks), (j / KS) & 1, abort_flag)) return false;
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k)
-          umma_bf16(t_s(j), kmajor_desc(base + L::Q, k), kmajor_desc(base + L::K + ks * L::TILE, k), idesc_s, k != 0);
+          umma_bf16_elect(leader, t_s(j), kmajor_desc(base + L::Q, k), kmajor_desc(base + L::K + ks * L::TILE, k), idesc_s, k != 0);
         return true;
       };
       auto issue_dp = [&](int j) -> bool {  // dP(j) = dO V_j^T; with it the inputs of softmax(j) are complete
         const int vs = j % VS;
-        if (!mbar_wait(bar(TQ_V_FULL0 + vs), (j / VS) & 1, abort_flag)) return false;
+        if (!mbar_wait_warp(bar(TQ_V_FULL0 + vs), (j / VS) & 1, abort_flag)) return false;
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k)
-          umma_bf16(t_dp, kmajor_desc(base + L::DO, k), kmajor_desc(base + L::V + vs * L::TILE, k), idesc_s, k != 0);
-        umma_commit(bar(TQ_SDP_FULL));
-        umma_commit(bar(TQ_V_EMPTY0 + vs));
+          umma_bf16_elect(leader, t_dp, kmajor_desc(base + L::DO, k), kmajor_desc(base + L::V + vs * L::TILE, k), idesc_s, k != 0);
+        umma_commit_elect(leader, bar(TQ_SDP_FULL));
+        umma_commit_elect(leader, bar(TQ_V_EMPTY0 + vs));
         return true;
       };
-      bool ok = mbar_wait(bar(TQ_QDO_FULL), 0, abort_flag);
+      bool ok = mbar_wait_warp(bar(TQ_QDO_FULL), 0, abort_flag);
       if (ok) ok = issue_s(0) && issue_dp(0);
       if (ok && n_kv > 1) ok = issue_s(1);
       for (int j = 0; j < n_kv && ok; ++j) {
         if (j + 1 < n_kv) {
           // the softmax threads hold S(j) and dP(j) in registers: the dP region may be overwritten
-          if (!mbar_wait(bar(TQ_LOADED), j & 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(bar(TQ_LOADED), j & 1, abort_flag)) { ok = false; break; }
           if (!issue_dp(j + 1)) { ok = false; break; }
         }
-        if (!mbar_wait(bar(TQ_DS_READY), j & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(TQ_DS_READY), j & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         // dQ += dS K_j   (contraction over the 128 key rows; A = dS from tensor memory)
         const uint32_t sk = base + L::K + (j % KS) * L::TILE;
 #pragma unroll
         for (int k = 0; k < BLK / 16; ++k)
-          umma_bf16_ts(t_dq, packed_kstep(t_s(j), k), mnmajor_desc(sk, k), idesc_q, (j | k) != 0);
-        umma_commit(bar(TQ_K_EMPTY0 + (j % KS)));
+          umma_bf16_ts_elect(leader, t_dq, packed_kstep(t_s(j), k), mnmajor_desc(sk, k), idesc_q, (j | k) != 0);
+        umma_commit_elect(leader, bar(TQ_K_EMPTY0 + (j % KS)));
         // the score region of tile j is free again once those MMAs have run (in order): tile j+2 goes there
         if (j + 2 < n_kv && !issue_s(j + 2)) { ok = false; break; }
       }
-      if (ok) umma_commit(bar(TQ_DONE));
+      if (ok) umma_commit_elect(leader, bar(TQ_DONE));
     }
   } else {
     const int q = warp & 3;
@@ -260,57 +261,64 @@ int launch_dq_tmem(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorM
 // directly and runs under the formation of dS(t); dP(t + 1) comes last, where nobody waits for it.  Head dimension 64
 // leaves room for two score regions (LA = 2): the scores of the next item are then ready before they are asked for.
 // With head dimension 128 the two accumulators take half of the tensor memory and LA is 1.
+// There the softmax threads set the pace, so two groups of eight warps take turns on the items; with head dimension 128
+// one group has the registers it needs and the score region is the limit.
 // What bounds it: the exponentials of an item take 1024 cycles of the MUFU unit (16 a cycle and SM) and the softmax threads
-// about as long again for loads, dS, packing and stores; the four products take 2048 cycles at head dimension 128 and
-// 1024 at 64.  Measured against attn_dkdv_split_kernel (P and dS through shared memory): 233 us for 275 (one sequence of
-// 4096, 32/8 heads of 128), 104 for 129 (two of 2048, 32/8 heads of 64).  At head dimension 128 the tensor pipe is issued
-// to without a break (80 to 108 cycles an instruction, 64 nominal: the operands of S and dP come from shared memory at
-// its full rate); at 64 the softmax threads set the pace.
+// about half as long again for loads, dS, packing and stores; the four products take 2048 cycles at head dimension 128 and
+// 1024 at 64.  An item takes 2750 cycles (128: exponentials, then the last half of dV and the next S behind each other)
+// and 2300 (64: dS, dK and the next dP behind each other).  Measured, with the MMA warp as it is now and before it
+// stayed converged, and for attn_dkdv_split_kernel (P and dS through shared memory): 214, 233 and 275 us (one sequence
+// of 4096, 32/8 heads of 128); 92, 104 and 129 us (two of 2048, 32/8 heads of 64).
 template <int HD>
 struct DkvTmemSmem {
   static constexpr int LA = HD == 64 ? 2 : 1;  // score regions: how many items ahead S is issued
   static constexpr int QST = LA + 1;           // Q(t) is read by dK(t) after S(t + LA) has been issued
   static constexpr int DST = 2;
+  static constexpr int NG = LA;                // groups of 8 softmax warps that take turns
+  static constexpr int THREADS = 64 + NG * 256;
   static constexpr uint32_t TILE = BLK * HD * 2;
   static constexpr uint32_t K = 0, V = TILE, Q = 2 * TILE, DO = Q + QST * TILE;
-  static constexpr uint32_t STATS = DO + DST * TILE;  // float [2 buffers][lse 128 | delta 128]
-  static constexpr uint32_t BARS = STATS + 2 * 2 * BLK * 4;
+  static constexpr uint32_t STATS = DO + DST * TILE;  // float [groups][2 buffers][lse 128 | delta 128]
+  static constexpr uint32_t BARS = STATS + NG * 2 * 2 * BLK * 4;
   static constexpr uint32_t TOTAL = BARS + 256 + 1024;
 };
 enum DkvTmemBar {
   TK_KV_FULL = 0, TK_Q_FULL0, TK_Q_EMPTY0 = TK_Q_FULL0 + 3, TK_DO_FULL0 = TK_Q_EMPTY0 + 3, TK_DO_EMPTY0 = TK_DO_FULL0 + 2,
-  TK_S_FULL0 = TK_DO_EMPTY0 + 2, TK_DP_FULL = TK_S_FULL0 + 2, TK_P_LO, TK_P_HI, TK_DS_LO, TK_DS_HI, TK_ACC_DONE, NUM_TK_BARS
+  TK_S_FULL0 = TK_DO_EMPTY0 + 2, TK_DP_FULL0 = TK_S_FULL0 + 2,
+  // one of each per group of softmax warps: P and dS of the first and of the last 64 query columns are stored
+  TK_P_LO0 = TK_DP_FULL0 + 2, TK_P_HI0 = TK_P_LO0 + 2, TK_DS_LO0 = TK_P_HI0 + 2, TK_DS_HI0 = TK_DS_LO0 + 2,
+  TK_ACC_DONE = TK_DS_HI0 + 2, NUM_TK_BARS
 };
 
 // Column of k-step kk (16 of an item's 128 query columns) inside a 128-column region.  The thread of half h of a key row
 // owns columns [32 h, 32 h + 32) and [64 + 32 h, 64 + 32 h + 32) and packs each 32 values into the first 16 of their columns.
 __device__ __forceinline__ uint32_t dkv_kstep(uint32_t region, int kk) { return region + (kk >> 1) * 32 + (kk & 1) * 8; }
 
-// Barrier over the 256 softmax threads that tells all of them whether any passed `mine`.
-__device__ __forceinline__ bool softmax_threads_any(bool mine) {
+// Barrier over the 256 softmax threads of a group that tells all of them whether any passed `mine`.
+__device__ __forceinline__ bool softmax_threads_any(int group, bool mine) {
   uint32_t any;
   asm volatile(
       "{\n\t"
       ".reg .pred p, q;\n\t"
       "setp.ne.u32 p, %1, 0;\n\t"
-      "barrier.cta.red.or.pred.aligned q, 1, 256, p;\n\t"
+      "barrier.cta.red.or.pred.aligned q, %2, 256, p;\n\t"
       "selp.u32 %0, 1, 0, q;\n\t"
       "}\n"
       : "=r"(any)
-      : "r"(mine ? 1u : 0u)
+      : "r"(mine ? 1u : 0u), "r"(1 + group)
       : "memory");
   return any != 0;
 }
 
 template <int HD>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(DkvTmemSmem<HD>::THREADS, 1)
 attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                       const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                       const float* __restrict__ LSE, const float* __restrict__ delta, __nv_bfloat16* __restrict__ dK,
                       __nv_bfloat16* __restrict__ dV, int S, int Hq, int Hkv, long long lddk, long long lddv, float scale,
                       float scale_log2, int* status) {
   using L = DkvTmemSmem<HD>;
-  constexpr int LA = L::LA, QST = L::QST, DST = L::DST;
+  constexpr int LA = L::LA, QST = L::QST, DST = L::DST, NG = L::NG;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -321,7 +329,7 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::BARS + 8 * NUM_TK_BARS + 8);
   float* stats = reinterpret_cast<float*>(smem + L::STATS);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   const int n_tiles = (S + BLK - 1) / BLK;
   const int jt = blockIdx.x / Hkv;  // key tile; early key tiles have the most work and come first
   const int kv_head = blockIdx.x % Hkv, batch = blockIdx.y;
@@ -329,7 +337,7 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
   const int n_items = G * (n_tiles - jt);  // (query head of the group, query tile at or after the key tile)
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < NUM_TK_BARS; ++i) mbar_init(bar(i), (i >= TK_P_LO && i <= TK_DS_HI) ? 8 : 1);  // one arrival per softmax warp
+    for (int i = 0; i < NUM_TK_BARS; ++i) mbar_init(bar(i), (i >= TK_P_LO0 && i < TK_ACC_DONE) ? 8 : 1);  // one arrival per warp of a group
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tq);
@@ -370,28 +378,29 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const uint32_t leader = elect_one();
       constexpr uint32_t idesc_s = make_idesc_bf16(BLK, BLK, false, false);  // 128 keys x 128 queries
       constexpr uint32_t idesc_g = make_idesc_bf16(BLK, HD, false, true);
       // S^T = K Q^T of item t: the key tile is the A operand, so keys land on the lanes
       auto issue_s = [&](int t) -> bool {
         const int qs = t % QST;
-        if (!mbar_wait(bar(TK_Q_FULL0 + qs), (t / QST) & 1, abort_flag)) return false;
+        if (!mbar_wait_warp(bar(TK_Q_FULL0 + qs), (t / QST) & 1, abort_flag)) return false;
         tc_fence_after();
         const uint32_t sq = base + L::Q + qs * L::TILE;
 #pragma unroll
-        for (int k = 0; k < HD / 16; ++k) umma_bf16(t_st(t), kmajor_desc(base + L::K, k), kmajor_desc(sq, k), idesc_s, k != 0);
-        umma_commit(bar(TK_S_FULL0 + t % LA));
+        for (int k = 0; k < HD / 16; ++k) umma_bf16_elect(leader, t_st(t), kmajor_desc(base + L::K, k), kmajor_desc(sq, k), idesc_s, k != 0);
+        umma_commit_elect(leader, bar(TK_S_FULL0 + t % LA));
         return true;
       };
       auto issue_dp = [&](int t) -> bool {  // dP^T = V dO^T of item t
         const int ds = t % DST;
-        if (!mbar_wait(bar(TK_DO_FULL0 + ds), (t / DST) & 1, abort_flag)) return false;
+        if (!mbar_wait_warp(bar(TK_DO_FULL0 + ds), (t / DST) & 1, abort_flag)) return false;
         tc_fence_after();
         const uint32_t sdo = base + L::DO + ds * L::TILE;
 #pragma unroll
-        for (int k = 0; k < HD / 16; ++k) umma_bf16(t_dpt, kmajor_desc(base + L::V, k), kmajor_desc(sdo, k), idesc_s, k != 0);
-        umma_commit(bar(TK_DP_FULL));
+        for (int k = 0; k < HD / 16; ++k) umma_bf16_elect(leader, t_dpt, kmajor_desc(base + L::V, k), kmajor_desc(sdo, k), idesc_s, k != 0);
+        umma_commit_elect(leader, bar(TK_DP_FULL0 + t % NG));
         return true;
       };
       // acc (+)= A B over the item's query rows [64 half, 64 half + 64): A = P^T or dS^T from tensor memory
@@ -399,40 +408,43 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
 #pragma unroll
         for (int kk = 0; kk < 4; ++kk) {
           const int k = half * 4 + kk;
-          umma_bf16_ts(acc, dkv_kstep(a_region, k), mnmajor_desc(b_tile, k), idesc_g, (t | k) != 0);
+          umma_bf16_ts_elect(leader, acc, dkv_kstep(a_region, k), mnmajor_desc(b_tile, k), idesc_g, (t | k) != 0);
         }
       };
-      bool ok = mbar_wait(bar(TK_KV_FULL), 0, abort_flag);
+      bool ok = mbar_wait_warp(bar(TK_KV_FULL), 0, abort_flag);
       if (ok && n_items > 0) ok = issue_s(0) && issue_dp(0);
       if (ok && LA == 2 && n_items > 1) ok = issue_s(1);
       for (int t = 0; t < n_items && ok; ++t) {
-        const int qs = t % QST, ds = t % DST;
+        const int qs = t % QST, ds = t % DST, g = t % NG;
+        const uint32_t ph = (t / NG) & 1;
         const uint32_t sq = base + L::Q + qs * L::TILE, sdo = base + L::DO + ds * L::TILE;
-        if (!mbar_wait(bar(TK_P_LO), t & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(TK_P_LO0 + g), ph, abort_flag)) { ok = false; break; }
         tc_fence_after();
         issue_grad(t_dv, t_st(t), sdo, t, 0);
-        if (!mbar_wait(bar(TK_P_HI), t & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(TK_P_HI0 + g), ph, abort_flag)) { ok = false; break; }
         tc_fence_after();
         issue_grad(t_dv, t_st(t), sdo, t, 1);
-        umma_commit(bar(TK_DO_EMPTY0 + ds));
+        umma_commit_elect(leader, bar(TK_DO_EMPTY0 + ds));
         // in order behind dV(t), which was the last reader of the region
         if (t + LA < n_items && !issue_s(t + LA)) { ok = false; break; }
-        if (!mbar_wait(bar(TK_DS_LO), t & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(TK_DS_LO0 + g), ph, abort_flag)) { ok = false; break; }
         tc_fence_after();
         issue_grad(t_dk, t_dpt, sq, t, 0);
-        if (!mbar_wait(bar(TK_DS_HI), t & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(TK_DS_HI0 + g), ph, abort_flag)) { ok = false; break; }
         tc_fence_after();
         issue_grad(t_dk, t_dpt, sq, t, 1);
-        umma_commit(bar(TK_Q_EMPTY0 + qs));
+        umma_commit_elect(leader, bar(TK_Q_EMPTY0 + qs));
         if (t + 1 < n_items && !issue_dp(t + 1)) { ok = false; break; }
       }
-      if (ok) umma_commit(bar(TK_ACC_DONE));
+      if (ok) umma_commit_elect(leader, bar(TK_ACC_DONE));
     }
   } else {
     const int q = warp & 3;
-    const int hf = (warp - 2) >> 2;  // two threads per key row, each with 32 of the first and 32 of the last 64 query columns
+    const int g = (warp - 2) >> 3;          // group: takes the items t with t % NG == g
+    const int gw = (warp - 2) & 7;          // warp inside the group
+    const int hf = gw >> 2;          // two threads per key row, each with 32 of the first and 32 of the last 64 query columns
     const int r = q * 32 + lane;     // key row inside the tile
-    const int e = (warp - 2) * 32 + lane;  // 0..255: which statistic this thread fetches per item
+    const int e = gw * 32 + lane;    // 0..255: which statistic this thread fetches per item
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     bool ok = true;
     // statistic of a query tile for this thread's slot: log-sum-exp (slots 0..127) or delta (128..255) of one
@@ -444,21 +456,27 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
       return qrow < S ? delta[at] : 0.f;
     };
     int it = jt, head = kv_head * G;
-    float next_stat = n_items > 0 ? fetch_stat(head, it) : 0.f;
-    for (int t = 0; t < n_items; ++t) {
-      const bool diag = it == jt;
-      const int q_end = S - it * BLK;                  // query columns at or beyond this one do not exist
-      const bool masked = diag || q_end < BLK;         // the same for the whole block
-      float* my_stats = stats + (t & 1) * 2 * BLK;
-      my_stats[e] = next_stat;
+    auto advance = [&]() {
       if (++it == n_tiles) {
         it = jt;
         ++head;
       }
-      if (t + 1 < n_items) next_stat = fetch_stat(head, it);  // travels while this item is processed
+    };
+    if (g == 1) advance();
+    float next_stat = g < n_items ? fetch_stat(head, it) : 0.f;
+    for (int t = g; t < n_items; t += NG) {
+      const uint32_t ph = (t / NG) & 1;
+      const bool diag = it == jt;
+      const int q_end = S - it * BLK;                  // query columns at or beyond this one do not exist
+      const bool masked = diag || q_end < BLK;         // the same for the whole block
+      float* my_stats = stats + (g * 2 + ph) * 2 * BLK;
+      my_stats[e] = next_stat;
+#pragma unroll
+      for (int i = 0; i < NG; ++i) advance();
+      if (t + NG < n_items) next_stat = fetch_stat(head, it);  // travels while this item is processed
       ok = __all_sync(0xffffffffu, mbar_wait(bar(TK_S_FULL0 + t % LA), (t / LA) & 1, abort_flag)) && ok;
-      // every statistic of this item is in shared memory; all 256 threads leave together if one of them gave up
-      ok = !softmax_threads_any(!ok);
+      // every statistic of this item is in shared memory; all threads of the group leave together if one of them gave up
+      ok = !softmax_threads_any(g, !ok);
       if (!ok) break;
       tc_fence_after();
       float p[2][32];
@@ -488,44 +506,59 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();  // the lanes' stores are ordered before the one arrival of the warp
-          if (lane == 0) mbar_arrive(bar(h == 0 ? TK_P_LO : TK_P_HI));
+          if (lane == 0) mbar_arrive(bar((h == 0 ? TK_P_LO0 : TK_P_HI0) + g));
         }
       }
-      ok = __all_sync(0xffffffffu, mbar_wait(bar(TK_DP_FULL), t & 1, abort_flag));  // acted upon at the next item's barrier
+      ok = __all_sync(0xffffffffu, mbar_wait(bar(TK_DP_FULL0 + g), ph, abort_flag));  // acted upon at the next item's barrier
       tc_fence_after();
       {
-        uint32_t dv[2][32];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) tmem_ld_32x32(t_dpt + lane_addr + h * 64 + hf * 32, dv[h]);
-        tmem_ld_wait();
+        // one group: all of dP in flight at once.  Two groups have 96 registers a thread, so 16 columns at a time; the other
+        // group's work hides the waits.
+        constexpr int STEP = NG == 1 ? 64 : 16;
+        uint32_t dv[STEP];
+        if constexpr (NG == 1) {
+          tmem_ld_32x32(t_dpt + lane_addr + hf * 32, *reinterpret_cast<uint32_t(*)[32]>(&dv[0]));
+          tmem_ld_32x32(t_dpt + lane_addr + 64 + hf * 32, *reinterpret_cast<uint32_t(*)[32]>(&dv[32]));
+          tmem_ld_wait();
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int c0 = h * 64 + hf * 32;
+          uint32_t packed[16];
 #pragma unroll
           for (int i4 = 0; i4 < 8; ++i4) {
+            if constexpr (NG == 2) {
+              if (i4 % 4 == 0) {
+                tmem_ld_32x16(t_dpt + lane_addr + c0 + i4 * 4, *reinterpret_cast<uint32_t(*)[16]>(&dv[0]));
+                tmem_ld_wait();
+              }
+            }
             const float4 dl = *reinterpret_cast<const float4*>(my_stats + BLK + c0 + i4 * 4);
             const float dlv[4] = {dl.x, dl.y, dl.z, dl.w};
+            float ds[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) p[h][i4 * 4 + u] *= __uint_as_float(dv[h][i4 * 4 + u]) - dlv[u];
+            for (int u = 0; u < 4; ++u) ds[u] = p[h][i4 * 4 + u] * (__uint_as_float(dv[(h * 32 + i4 * 4 + u) % STEP]) - dlv[u]);
+            packed[i4 * 2] = pack_bf16(ds[0], ds[1]);
+            packed[i4 * 2 + 1] = pack_bf16(ds[2], ds[3]);
           }
-          uint32_t packed[16];
-          pack32(p[h], packed);
           tmem_st_32x16(t_dpt + lane_addr + c0, packed);
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(bar(h == 0 ? TK_DS_LO : TK_DS_HI));
+          if (lane == 0) mbar_arrive(bar((h == 0 ? TK_DS_LO0 : TK_DS_HI0) + g));
         }
       }
     }
-    if (ok && n_items > 0) {
+    if (ok) {
       const bool done = mbar_wait(bar(TK_ACC_DONE), 0, abort_flag);
       if (__all_sync(0xffffffffu, done)) {
         tc_fence_after();
         const int krow = jt * BLK + r;
         const long long tok = static_cast<long long>(batch) * S + krow;
-        store_acc<HD / 2>(t_dv + lane_addr + hf * (HD / 2), dV + tok * lddv + kv_head * HD + hf * (HD / 2), 1.f, krow < S);
-        store_acc<HD / 2>(t_dk + lane_addr + hf * (HD / 2), dK + tok * lddk + kv_head * HD + hf * (HD / 2), scale, krow < S);
+        if (NG == 1 || g == 0)
+          store_acc<HD / 2>(t_dv + lane_addr + hf * (HD / 2), dV + tok * lddv + kv_head * HD + hf * (HD / 2), 1.f, krow < S);
+        if (NG == 1 || g == 1)
+          store_acc<HD / 2>(t_dk + lane_addr + hf * (HD / 2), dK + tok * lddk + kv_head * HD + hf * (HD / 2), scale, krow < S);
       }
     }
     tc_fence_before();
@@ -556,7 +589,7 @@ int launch_dkdv_tmem(const CUtensorMap& tq, const CUtensorMap& tk, const CUtenso
     configured = true;
   }
   const int n_tiles = (S + BLK - 1) / BLK;
-  attn_dkdv_tmem_kernel<HD><<<dim3(n_tiles * Hkv, B, 1), 320, DkvTmemSmem<HD>::TOTAL, stream>>>(
+  attn_dkdv_tmem_kernel<HD><<<dim3(n_tiles * Hkv, B, 1), DkvTmemSmem<HD>::THREADS, DkvTmemSmem<HD>::TOTAL, stream>>>(
       tq, tk, tv, tdo, lse, delta, static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), S, Hq, Hkv, lddk,
       lddv, scale, scale * 1.4426950408889634f, status);
   return static_cast<int>(cudaGetLastError());

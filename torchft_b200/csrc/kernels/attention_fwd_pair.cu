@@ -145,7 +145,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
   volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(smem + L::BARS + 8 * NUM_PAIR_BARS);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::BARS + 8 * NUM_PAIR_BARS + 8);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   const int n_qtiles = (S + BLK - 1) / BLK;
   const int n_pairs = (n_qtiles + 1) / 2;
   const int pair = n_pairs - 1 - blockIdx.x / Hq;  // heaviest pairs first, over all heads
@@ -194,16 +194,17 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
+      const uint32_t leader = elect_one();
       constexpr uint32_t idesc_s = make_idesc_bf16(BLK, BLK, false, false);
       constexpr uint32_t idesc_pv = make_idesc_bf16(BLK, HD, false, true);
       auto issue_s = [&](int t, int j) {
         const int st = j & 1;
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k)
-          umma_bf16(tmem_s(t), kmajor_desc(base + L::Q + t * L::TILE, k), kmajor_desc(base + L::K + st * L::TILE, k),
+          umma_bf16_elect(leader, tmem_s(t), kmajor_desc(base + L::Q + t * L::TILE, k), kmajor_desc(base + L::K + st * L::TILE, k),
                     idesc_s, k != 0);
-        umma_commit(bar(PS_FULL_A + t));
+        umma_commit_elect(leader, bar(PS_FULL_A + t));
       };
       // the PV product over keys [64 half, 64 half + 64) of the tile: 16 keys per step = 8 packed columns of P
       auto issue_pv = [&](int t, int j, int half) {
@@ -211,47 +212,47 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
 #pragma unroll
         for (int kk = 0; kk < BLK / 32; ++kk) {
           const int k = half * (BLK / 32) + kk;
-          umma_bf16_ts(tmem_o(t), tmem_s(t) + k * 8, mnmajor_desc(base + L::V + st * L::TILE, k), idesc_pv,
+          umma_bf16_ts_elect(leader, tmem_o(t), tmem_s(t) + k * 8, mnmajor_desc(base + L::V + st * L::TILE, k), idesc_pv,
                        (j > 0 || k > 0) ? 1u : 0u);
         }
       };
       // P of the first 64 keys is ready before the exponentials of the last 64 are: start on it
       auto wait_issue_pv = [&](int t, int j) {
-        if (!mbar_wait(bar(PP_LO_A + t), j & 1, abort_flag)) return false;
+        if (!mbar_wait_warp(bar(PP_LO_A + t), j & 1, abort_flag)) return false;
         tc_fence_after();
         issue_pv(t, j, 0);
-        if (!mbar_wait(bar(PP_HI_A + t), j & 1, abort_flag)) return false;
+        if (!mbar_wait_warp(bar(PP_HI_A + t), j & 1, abort_flag)) return false;
         tc_fence_after();
         issue_pv(t, j, 1);
         return true;
       };
-      bool ok = mbar_wait(bar(PQ_FULL), 0, abort_flag) && mbar_wait(bar(PK_FULL0), 0, abort_flag);
+      bool ok = mbar_wait_warp(bar(PQ_FULL), 0, abort_flag) && mbar_wait_warp(bar(PK_FULL0), 0, abort_flag);
       if (ok) {
         tc_fence_after();
         issue_s(0, 0);
         if (has_b) issue_s(1, 0);
-        umma_commit(bar(PK_EMPTY0));
+        umma_commit_elect(leader, bar(PK_EMPTY0));
       }
       for (int j = 0; j < n_steps && ok; ++j) {
         const int st = j & 1;
-        if (!mbar_wait(bar(PV_FULL0 + st), (j >> 1) & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(PV_FULL0 + st), (j >> 1) & 1, abort_flag)) { ok = false; break; }
         if (j < n_a) {
           if (!wait_issue_pv(0, j)) { ok = false; break; }
-          if (j == n_a - 1) umma_commit(bar(PO_FULL_A));
+          if (j == n_a - 1) umma_commit_elect(leader, bar(PO_FULL_A));
         }
         const bool have_next = j + 1 < n_steps;
         if (have_next) {
-          if (!mbar_wait(bar(PK_FULL0 + ((j + 1) & 1)), ((j + 1) >> 1) & 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(bar(PK_FULL0 + ((j + 1) & 1)), ((j + 1) >> 1) & 1, abort_flag)) { ok = false; break; }
           tc_fence_after();
         }
         if (j + 1 < n_a) issue_s(0, j + 1);
         if (j < n_b) {
           if (!wait_issue_pv(1, j)) { ok = false; break; }
-          if (j == n_b - 1) umma_commit(bar(PO_FULL_B));
+          if (j == n_b - 1) umma_commit_elect(leader, bar(PO_FULL_B));
         }
-        umma_commit(bar(PV_EMPTY0 + st));
+        umma_commit_elect(leader, bar(PV_EMPTY0 + st));
         if (j + 1 < n_b) issue_s(1, j + 1);
-        if (have_next) umma_commit(bar(PK_EMPTY0 + ((j + 1) & 1)));
+        if (have_next) umma_commit_elect(leader, bar(PK_EMPTY0 + ((j + 1) & 1)));
       }
     }
   } else {

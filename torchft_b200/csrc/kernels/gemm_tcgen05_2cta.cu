@@ -78,24 +78,30 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols));
 }
-__device__ __forceinline__ void umma_bf16_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                               uint32_t accumulate) {
+// Issued by the lane that `leader` names; the warp stays converged (umma_bf16_elect in common.cuh says why).
+__device__ __forceinline__ void umma_bf16_pair(uint32_t leader, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
+                                               uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t"
-      ".reg .pred p;\n\t"
+      ".reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
       "}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader)
       : "memory");
 }
 // Arrives on the barrier at the same shared-memory offset in BOTH CTAs of the pair once every MMA
 // issued so far by this thread has retired.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
+__device__ __forceinline__ void umma_commit_pair(uint32_t leader, uint32_t bar) {
   const uint16_t mask = 3;
   asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-      "h"(mask)
+      "{\n\t"
+      ".reg .pred q;\n\t"
+      "setp.ne.b32 q, %2, 0;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t"
+      "}\n" ::"r"(bar),
+      "h"(mask), "r"(leader)
       : "memory");
 }
 
@@ -216,7 +222,7 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
   volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(bars + 2 * STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * STAGES + 5);
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = uniform_warp_index();
   const int lane = threadIdx.x & 31;
   const uint32_t cta = cluster_ctarank();  // 0: leader of the pair
   const int pair = blockIdx.x >> 1;
@@ -282,7 +288,8 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && cta == 0) {
+    if (cta == 0) {
+      const uint32_t leader = elect_one();
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -291,11 +298,11 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
         const Unit un = unit_at(sched, u);
         const uint32_t idesc = un.ncols == BN ? make_idesc_bf16(BM, BN, A_MN, B_MN) : make_idesc_bf16(BM, BN / 2, A_MN, B_MN);
         const int buf = it & 1;
-        if (!mbar_wait(tempty_bar(buf), (((it >> 1) & 1) ^ 1), abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(tempty_bar(buf), (((it >> 1) & 1) ^ 1), abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * BN;
         for (int kb = 0; kb < kblocks; ++kb) {
-          if (!mbar_wait(full_bar(stage), phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(full_bar(stage), phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = base + stage * STAGE_BYTES;
           const uint32_t sb = sa + A_STAGE_BYTES;
@@ -303,12 +310,12 @@ gemm2_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ 
           for (int k = 0; k < BK / UMMA_K; ++k) {
             const uint64_t adesc = A_MN ? make_smem_desc(sa + k * 2048, 8192, 1024) : make_smem_desc(sa + k * 32, 16, 1024);
             const uint64_t bdesc = B_MN ? make_smem_desc(sb + k * 2048, 8192, 1024) : make_smem_desc(sb + k * 32, 16, 1024);
-            umma_bf16_pair(d_tmem, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
+            umma_bf16_pair(leader, d_tmem, adesc, bdesc, idesc, (kb | k) != 0 ? 1u : 0u);
           }
-          umma_commit_pair(empty_bar(stage));
+          umma_commit_pair(leader, empty_bar(stage));
           if (++stage == STAGES) { stage = 0; phase ^= 1u; }
         }
-        if (ok) umma_commit_pair(tfull_bar(buf));
+        if (ok) umma_commit_pair(leader, tfull_bar(buf));
       }
     }
   } else {
