@@ -217,8 +217,8 @@ attn_dkdv_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__
       tc_fence_after();
       const int krow = jt * BLK + r;
       const long long tok = static_cast<long long>(batch) * S + krow;
-      store_acc<HD / 2>(t_dv + lane_addr + half * (HD / 2), dV + tok * lddv + kv_head * HD + half * (HD / 2), 1.f, krow < S);
-      store_acc<HD / 2>(t_dk + lane_addr + half * (HD / 2), dK + tok * lddk + kv_head * HD + half * (HD / 2), scale, krow < S);
+      store_acc<HD / 2>(t_dv + lane_addr + half * (HD / 2), dV + tok * lddv + kv_head * HD + half * (HD / 2), lddv, 1.f, S - krow);
+      store_acc<HD / 2>(t_dk + lane_addr + half * (HD / 2), dK + tok * lddk + kv_head * HD + half * (HD / 2), lddk, scale, S - krow);
     }
     tc_fence_before();
   }
@@ -464,8 +464,8 @@ attn_dkdv_split_kernel(const __grid_constant__ CUtensorMap tq, const __grid_cons
       tc_fence_after();
       const int krow = jt * BLK + r;
       const long long tok = static_cast<long long>(batch) * S + krow;
-      store_acc<HD / 2>(t_dv + lane_addr + half * (HD / 2), dV + tok * lddv + kv_head * HD + half * (HD / 2), 1.f, krow < S);
-      store_acc<HD / 2>(t_dk + lane_addr + half * (HD / 2), dK + tok * lddk + kv_head * HD + half * (HD / 2), scale, krow < S);
+      store_acc<HD / 2>(t_dv + lane_addr + half * (HD / 2), dV + tok * lddv + kv_head * HD + half * (HD / 2), lddv, 1.f, S - krow);
+      store_acc<HD / 2>(t_dk + lane_addr + half * (HD / 2), dK + tok * lddk + kv_head * HD + half * (HD / 2), lddk, scale, S - krow);
     }
     tc_fence_before();
   }
@@ -642,7 +642,7 @@ attn_dq_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ C
     if (ok && mbar_wait(bar(DQ_DONE), 0, abort_flag)) {
       tc_fence_after();
       const long long tok = static_cast<long long>(batch) * S + row;
-      store_acc<HD / 2>(t_dq + lane_addr + half * (HD / 2), dQ + tok * lddq + head * HD + half * (HD / 2), scale, row_ok);
+      store_acc<HD / 2>(t_dq + lane_addr + half * (HD / 2), dQ + tok * lddq + head * HD + half * (HD / 2), lddq, scale, S - row);
     }
     tc_fence_before();
   }
@@ -683,10 +683,7 @@ int launch_bwd(const void* dout, const void* q, const void* k, const void* v, co
   }
   cudaGetLastError();
   const float scale_log2 = scale * 1.4426950408889634f;
-  const long long warps = static_cast<long long>(B) * S * Hq;
-  if (parts & 1)
-    attn_delta_kernel<HD><<<static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(dout), delta, B, S, Hq);
+  if (parts & 1) launch_delta<HD>(o, dout, delta, B, S, Hq, stream);
   const int n_tiles = (S + BLK - 1) / BLK;
   if ((parts & 2) && (parts & 8))
     attn_dkdv_split_kernel<HD><<<dim3(n_tiles * Hkv, B, 1), 320, DkvSmem<HD>::TOTAL, stream>>>(

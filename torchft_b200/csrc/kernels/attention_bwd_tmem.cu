@@ -6,7 +6,7 @@
 // handshake per operand.  Here they are written with tcgen05.st over the fp32 values they were
 // computed from and consumed by the gradient MMAs as the A operand FROM tensor memory:
 //
-//   attn_dq_tmem_kernel     one CTA per (query tile, head).  S = Q K_j^T alternates between two score
+//   attn_dq_tmem_kernel     work items (query tile, head).  S = Q K_j^T alternates between two score
 //                           regions, dP = dO V_j^T has one.  The softmax threads pull both into
 //                           registers (all loads in flight, one wait), report that (the dP region is
 //                           then free for tile j+1), form dS = P (dP - delta) and store it, packed,
@@ -38,27 +38,56 @@ __device__ __forceinline__ uint32_t packed_kstep(uint32_t region, int k) {
 }
 
 // ------------------------------------------------------------------ dQ
+// Persistent: one CTA per SM walks over (query tile, head, batch) work items, heaviest first and in alternating direction
+// from round to round, which evens out the triangular lengths.  Loads of the next item's Q and dO start when the last
+// products that read the present ones have run, so they travel under the last softmax and the store of dQ.  With one
+// item per CTA (seven CTAs per SM at S 4096, 32 heads) launch, tensor-memory allocation, first loads and store cost 10.7
+// thousand cycles an item, a fifth of the time.  S 4096, 32/8 heads of 128: 156 us for 164; two of 2048, heads of 64: 69 for 82.
+// At head dimension 64 the softmax threads set the pace (1024 cycles of MUFU a tile against 768 of products), so two groups
+// of eight warps take turns on the key tiles, and Q, dO and the accumulator have two buffers: one group stores an item's
+// dQ while the other works on the next item.
 template <int HD>
 struct DqTmemSmem {
   static constexpr int KSTAGES = 3, VSTAGES = 2;
+  static constexpr int NG = HD == 64 ? 2 : 1;  // groups of 8 softmax warps
+  static constexpr int QB = HD == 64 ? 2 : 1;  // buffers of Q, dO and dQ
+  static constexpr int THREADS = 64 + NG * 256;
   static constexpr uint32_t TILE = BLK * HD * 2;
-  static constexpr uint32_t Q = 0, DO = TILE, K = 2 * TILE, V = K + KSTAGES * TILE;
+  static constexpr uint32_t Q = 0, DO = QB * TILE, K = 2 * QB * TILE, V = K + KSTAGES * TILE;
   static constexpr uint32_t BARS = V + VSTAGES * TILE;
   static constexpr uint32_t TOTAL = BARS + 256 + 1024;
 };
 enum DqTmemBar {
-  TQ_QDO_FULL = 0, TQ_K_FULL0, TQ_K_FULL1, TQ_K_FULL2, TQ_K_EMPTY0, TQ_K_EMPTY1, TQ_K_EMPTY2, TQ_V_FULL0, TQ_V_FULL1,
-  TQ_V_EMPTY0, TQ_V_EMPTY1, TQ_SDP_FULL, TQ_LOADED, TQ_DS_READY, TQ_DONE, NUM_TQ_BARS
+  TQ_QDO_FULL0 = 0, TQ_QDO_EMPTY0 = 2, TQ_K_FULL0 = 4, TQ_K_EMPTY0 = 7, TQ_V_FULL0 = 10, TQ_V_EMPTY0 = 12,
+  // by parity of the tile's number in this CTA: inputs complete / read into registers / dS stored
+  TQ_SDP_FULL0 = 14, TQ_LOADED0 = 16, TQ_DS_READY0 = 18,
+  TQ_DQ_EMPTY0 = 20, TQ_DQ_FULL0 = 22, NUM_TQ_BARS = 24
 };
+static_assert(8 * NUM_TQ_BARS + 16 <= 256, "barriers, tensor-memory address and abort flag share 256 bytes");
+
+struct DqItem {
+  int qt, head, batch;
+};
+// Item of round i for this CTA; -1 as query tile if there is none.
+__device__ __forceinline__ DqItem dq_item(int i, int n_tiles, int Hq, int B) {
+  const int G = gridDim.x, per_tile = Hq * B;
+  const int w = i * G + ((i & 1) ? G - 1 - static_cast<int>(blockIdx.x) : static_cast<int>(blockIdx.x));
+  DqItem it;
+  it.qt = w < n_tiles * per_tile ? n_tiles - 1 - w / per_tile : -1;
+  const int rest = w % per_tile;
+  it.head = rest % Hq;
+  it.batch = rest / Hq;
+  return it;
+}
 
 template <int HD>
-__global__ void __launch_bounds__(320, 1)
+__global__ void __launch_bounds__(DqTmemSmem<HD>::THREADS, 1)
 attn_dq_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
                     const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
                     const float* __restrict__ LSE, const float* __restrict__ delta, __nv_bfloat16* __restrict__ dQ,
-                    int S, int Hq, int Hkv, long long lddq, float scale, float scale_log2, int* status) {
+                    int B, int S, int Hq, int Hkv, long long lddq, float scale, float scale_log2, int* status) {
   using L = DqTmemSmem<HD>;
-  constexpr int KS = L::KSTAGES, VS = L::VSTAGES;
+  constexpr int KS = L::KSTAGES, VS = L::VSTAGES, NG = L::NG, QB = L::QB;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -70,13 +99,11 @@ attn_dq_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
 
   const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
   const int n_tiles = (S + BLK - 1) / BLK;
-  const int qt = n_tiles - 1 - blockIdx.x / Hq;  // heaviest first over all heads
-  const int head = blockIdx.x % Hq, batch = blockIdx.y;
-  const int kv_head = head / (Hq / Hkv);
-  const int n_kv = qt + 1;
+  const int group = Hq / Hkv;
+  const int rounds = (n_tiles * Hq * B + gridDim.x - 1) / gridDim.x;
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < NUM_TQ_BARS; ++i) mbar_init(bar(i), (i == TQ_LOADED || i == TQ_DS_READY) ? 256 : 1);
+    for (int i = 0; i < NUM_TQ_BARS; ++i) mbar_init(bar(i), (i >= TQ_LOADED0 && i < TQ_DQ_FULL0) ? 8 : 1);  // one arrival per warp of a group
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tq);
@@ -92,130 +119,177 @@ attn_dq_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  auto t_s = [&](int j) { return tmem_base + static_cast<uint32_t>(j & 1) * 128u; };  // scores, later dS, of tile j
-  const uint32_t t_dp = tmem_base + 256, t_dq = tmem_base + 384;
+  auto t_s = [&](int c) { return tmem_base + static_cast<uint32_t>(c & 1) * 128u; };  // scores, later dS, of tile c
+  const uint32_t t_dp = tmem_base + 256;
+  auto t_dq = [&](int u) { return tmem_base + 384u + static_cast<uint32_t>(u % QB) * HD; };
+  // u counts the items of this CTA, c its key tiles; both run on from item to item, and with them every barrier phase
 
   if (warp == 0) {
     if (lane == 0) {
-      mbar_expect_tx(bar(TQ_QDO_FULL), 2 * L::TILE);
-      load_tile<HD>(base + L::Q, &tq, bar(TQ_QDO_FULL), head, qt * BLK, batch);
-      load_tile<HD>(base + L::DO, &tdo, bar(TQ_QDO_FULL), head, qt * BLK, batch);
-      for (int j = 0; j < n_kv; ++j) {
-        const int ks = j % KS, vs = j % VS;
-        if (!mbar_wait(bar(TQ_K_EMPTY0 + ks), ((j / KS) & 1) ^ 1, abort_flag)) break;
-        mbar_expect_tx(bar(TQ_K_FULL0 + ks), L::TILE);
-        load_tile<HD>(base + L::K + ks * L::TILE, &tk, bar(TQ_K_FULL0 + ks), kv_head, j * BLK, batch);
-        if (!mbar_wait(bar(TQ_V_EMPTY0 + vs), ((j / VS) & 1) ^ 1, abort_flag)) break;
-        mbar_expect_tx(bar(TQ_V_FULL0 + vs), L::TILE);
-        load_tile<HD>(base + L::V + vs * L::TILE, &tv, bar(TQ_V_FULL0 + vs), kv_head, j * BLK, batch);
+      bool ok = true;
+      for (int i = 0, u = 0, c = 0; i < rounds && ok; ++i) {
+        const DqItem w = dq_item(i, n_tiles, Hq, B);
+        if (w.qt < 0) continue;
+        const int qb = u % QB, kv_head = w.head / group;
+        if (!mbar_wait(bar(TQ_QDO_EMPTY0 + qb), ((u / QB) & 1) ^ 1, abort_flag)) break;
+        mbar_expect_tx(bar(TQ_QDO_FULL0 + qb), 2 * L::TILE);
+        load_tile<HD>(base + L::Q + qb * L::TILE, &tq, bar(TQ_QDO_FULL0 + qb), w.head, w.qt * BLK, w.batch);
+        load_tile<HD>(base + L::DO + qb * L::TILE, &tdo, bar(TQ_QDO_FULL0 + qb), w.head, w.qt * BLK, w.batch);
+        for (int j = 0; j <= w.qt; ++j, ++c) {
+          const int ks = c % KS, vs = c % VS;
+          ok = mbar_wait(bar(TQ_K_EMPTY0 + ks), ((c / KS) & 1) ^ 1, abort_flag);
+          if (!ok) break;
+          mbar_expect_tx(bar(TQ_K_FULL0 + ks), L::TILE);
+          load_tile<HD>(base + L::K + ks * L::TILE, &tk, bar(TQ_K_FULL0 + ks), kv_head, j * BLK, w.batch);
+          ok = mbar_wait(bar(TQ_V_EMPTY0 + vs), ((c / VS) & 1) ^ 1, abort_flag);
+          if (!ok) break;
+          mbar_expect_tx(bar(TQ_V_FULL0 + vs), L::TILE);
+          load_tile<HD>(base + L::V + vs * L::TILE, &tv, bar(TQ_V_FULL0 + vs), kv_head, j * BLK, w.batch);
+        }
+        ++u;
       }
     }
   } else if (warp == 1) {
-    {
-      const uint32_t leader = elect_one();
-      constexpr uint32_t idesc_s = make_idesc_bf16(BLK, BLK, false, false);
-      constexpr uint32_t idesc_q = make_idesc_bf16(BLK, HD, false, true);
-      auto issue_s = [&](int j) -> bool {  // S(j) = Q K_j^T into the score region of tile j
-        const int ks = j % KS;
-        if (!mbar_wait_warp(bar(TQ_K_FULL0 + ks), (j / KS) & 1, abort_flag)) return false;
-        tc_fence_after();
+    const uint32_t leader = elect_one();
+    constexpr uint32_t idesc_s = make_idesc_bf16(BLK, BLK, false, false);
+    constexpr uint32_t idesc_q = make_idesc_bf16(BLK, HD, false, true);
+    auto issue_s = [&](int c, uint32_t sq) -> bool {  // S(c) = Q K^T into the score region of tile c
+      const int ks = c % KS;
+      if (!mbar_wait_warp(bar(TQ_K_FULL0 + ks), (c / KS) & 1, abort_flag)) return false;
+      tc_fence_after();
 #pragma unroll
-        for (int k = 0; k < HD / 16; ++k)
-          umma_bf16_elect(leader, t_s(j), kmajor_desc(base + L::Q, k), kmajor_desc(base + L::K + ks * L::TILE, k), idesc_s, k != 0);
-        return true;
-      };
-      auto issue_dp = [&](int j) -> bool {  // dP(j) = dO V_j^T; with it the inputs of softmax(j) are complete
-        const int vs = j % VS;
-        if (!mbar_wait_warp(bar(TQ_V_FULL0 + vs), (j / VS) & 1, abort_flag)) return false;
-        tc_fence_after();
+      for (int k = 0; k < HD / 16; ++k)
+        umma_bf16_elect(leader, t_s(c), kmajor_desc(sq, k), kmajor_desc(base + L::K + ks * L::TILE, k), idesc_s, k != 0);
+      return true;
+    };
+    // dP(c) = dO V^T, once the softmax threads hold dP(c - 1) in registers; with it the inputs of softmax(c) are complete
+    auto issue_dp = [&](int c, uint32_t sdo) -> bool {
+      const int vs = c % VS;
+      if (c > 0 && !mbar_wait_warp(bar(TQ_LOADED0 + ((c - 1) & 1)), ((c - 1) >> 1) & 1, abort_flag)) return false;
+      if (!mbar_wait_warp(bar(TQ_V_FULL0 + vs), (c / VS) & 1, abort_flag)) return false;
+      tc_fence_after();
 #pragma unroll
-        for (int k = 0; k < HD / 16; ++k)
-          umma_bf16_elect(leader, t_dp, kmajor_desc(base + L::DO, k), kmajor_desc(base + L::V + vs * L::TILE, k), idesc_s, k != 0);
-        umma_commit_elect(leader, bar(TQ_SDP_FULL));
-        umma_commit_elect(leader, bar(TQ_V_EMPTY0 + vs));
-        return true;
-      };
-      bool ok = mbar_wait_warp(bar(TQ_QDO_FULL), 0, abort_flag);
-      if (ok) ok = issue_s(0) && issue_dp(0);
-      if (ok && n_kv > 1) ok = issue_s(1);
+      for (int k = 0; k < HD / 16; ++k)
+        umma_bf16_elect(leader, t_dp, kmajor_desc(sdo, k), kmajor_desc(base + L::V + vs * L::TILE, k), idesc_s, k != 0);
+      umma_commit_elect(leader, bar(TQ_SDP_FULL0 + (c & 1)));
+      umma_commit_elect(leader, bar(TQ_V_EMPTY0 + vs));
+      return true;
+    };
+    bool ok = true;
+    for (int i = 0, u = 0, c0 = 0; i < rounds && ok; ++i) {
+      const DqItem w = dq_item(i, n_tiles, Hq, B);
+      if (w.qt < 0) continue;
+      const int qb = u % QB, n_kv = w.qt + 1;
+      const uint32_t sq = base + L::Q + qb * L::TILE, sdo = base + L::DO + qb * L::TILE, par = (u / QB) & 1;
+      ok = mbar_wait_warp(bar(TQ_QDO_FULL0 + qb), par, abort_flag) && issue_s(c0, sq) && issue_dp(c0, sdo);
+      if (ok && n_kv > 1) ok = issue_s(c0 + 1, sq);
+      if (ok && n_kv == 1) umma_commit_elect(leader, bar(TQ_QDO_EMPTY0 + qb));
       for (int j = 0; j < n_kv && ok; ++j) {
+        const int c = c0 + j;
         if (j + 1 < n_kv) {
-          // the softmax threads hold S(j) and dP(j) in registers: the dP region may be overwritten
-          if (!mbar_wait_warp(bar(TQ_LOADED), j & 1, abort_flag)) { ok = false; break; }
-          if (!issue_dp(j + 1)) { ok = false; break; }
+          if (!issue_dp(c + 1, sdo)) { ok = false; break; }
+          if (j + 2 == n_kv) umma_commit_elect(leader, bar(TQ_QDO_EMPTY0 + qb));  // nothing reads this Q and dO any more
         }
-        if (!mbar_wait_warp(bar(TQ_DS_READY), j & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(TQ_DS_READY0 + (c & 1)), (c >> 1) & 1, abort_flag)) { ok = false; break; }
+        if (j == 0 && !mbar_wait_warp(bar(TQ_DQ_EMPTY0 + qb), par ^ 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         // dQ += dS K_j   (contraction over the 128 key rows; A = dS from tensor memory)
-        const uint32_t sk = base + L::K + (j % KS) * L::TILE;
+        const uint32_t sk = base + L::K + (c % KS) * L::TILE;
 #pragma unroll
         for (int k = 0; k < BLK / 16; ++k)
-          umma_bf16_ts_elect(leader, t_dq, packed_kstep(t_s(j), k), mnmajor_desc(sk, k), idesc_q, (j | k) != 0);
-        umma_commit_elect(leader, bar(TQ_K_EMPTY0 + (j % KS)));
-        // the score region of tile j is free again once those MMAs have run (in order): tile j+2 goes there
-        if (j + 2 < n_kv && !issue_s(j + 2)) { ok = false; break; }
+          umma_bf16_ts_elect(leader, t_dq(u), packed_kstep(t_s(c), k), mnmajor_desc(sk, k), idesc_q, (j | k) != 0);
+        umma_commit_elect(leader, bar(TQ_K_EMPTY0 + (c % KS)));
+        // the score region of tile c is free again once those MMAs have run (in order): tile c + 2 goes there
+        if (j + 2 < n_kv && !issue_s(c + 2, sq)) { ok = false; break; }
       }
-      if (ok) umma_commit_elect(leader, bar(TQ_DONE));
+      if (ok) umma_commit_elect(leader, bar(TQ_DQ_FULL0 + qb));
+      c0 += n_kv;
+      ++u;
     }
   } else {
     const int q = warp & 3;
-    const int half = (warp - 2) >> 2;  // two threads per row: key columns [0,64) and [64,128)
+    const int g = (warp - 2) >> 3;           // group: takes the tiles c with c % NG == g
+    const int half = ((warp - 2) >> 2) & 1;  // two threads per row: key columns [0,64) and [64,128)
     const int r = q * 32 + lane;
-    const int row = qt * BLK + r;
-    const bool row_ok = row < S;
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
-    const long long stat = (static_cast<long long>(batch) * Hq + head) * S + row;
-    const float lse = row_ok ? LSE[stat] : 0.f;
-    const float dl = row_ok ? delta[stat] : 0.f;
     bool ok = true;
-    for (int j = 0; j < n_kv; ++j) {
-      const bool got = mbar_wait(bar(TQ_SDP_FULL), j & 1, abort_flag);
-      if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
-      tc_fence_after();
-      const bool diag = (j == qt);
-      const uint32_t my_s = t_s(j) + lane_addr + half * 64;
-      uint32_t sv[2][32], dv[2][32];
-#pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        tmem_ld_32x32(my_s + cc * 32, sv[cc]);
-        tmem_ld_32x32(t_dp + lane_addr + half * 64 + cc * 32, dv[cc]);
-      }
-      tmem_ld_wait();
-      tc_fence_before();
-      mbar_arrive(bar(TQ_LOADED));
-#pragma unroll
-      for (int cc = 0; cc < 2; ++cc) {
-        const int c0 = half * 64 + cc * 32;
-        float ds[32];
-        if (diag) {  // rows beyond the sequence need no mask: a row of dS reaches its own row of dQ only
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const bool keep = (c0 + i) <= r;
-            const float p = keep ? fast_exp2(__uint_as_float(sv[cc][i]) * scale_log2 - lse) : 0.f;
-            ds[i] = p * (__uint_as_float(dv[cc][i]) - dl);
-          }
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const float p = fast_exp2(__uint_as_float(sv[cc][i]) * scale_log2 - lse);
-            ds[i] = p * (__uint_as_float(dv[cc][i]) - dl);
-          }
-        }
-        uint32_t packed[16];
-        pack32(ds, packed);
-        tmem_st_32x16(my_s + cc * 16, packed);  // over score columns this thread has already read
-      }
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(bar(TQ_DS_READY));
-    }
-    if (ok) {
-      const bool done = mbar_wait(bar(TQ_DONE), 0, abort_flag);
-      if (__all_sync(0xffffffffu, done)) {
+    for (int i = 0, u = 0, c0 = 0; i < rounds && ok; ++i) {
+      const DqItem w = dq_item(i, n_tiles, Hq, B);
+      if (w.qt < 0) continue;
+      const int row = w.qt * BLK + r, n_kv = w.qt + 1;
+      const long long stat = (static_cast<long long>(w.batch) * Hq + w.head) * S + row;
+      const float lse = row < S ? LSE[stat] : 0.f;
+      const float dl = row < S ? delta[stat] : 0.f;
+      for (int j = NG == 1 ? 0 : (c0 + g) & 1; j < n_kv; j += NG) {
+        const int c = c0 + j;
+        if (!mbar_wait_warp(bar(TQ_SDP_FULL0 + (c & 1)), (c >> 1) & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        const long long tok = static_cast<long long>(batch) * S + row;
-        store_acc<HD / 2>(t_dq + lane_addr + half * (HD / 2), dQ + tok * lddq + head * HD + half * (HD / 2), scale, row_ok);
+        const bool diag = (j == w.qt);
+        const uint32_t my_s = t_s(c) + lane_addr + half * 64, my_dp = t_dp + lane_addr + half * 64;
+        auto loaded = [&]() {
+          tmem_ld_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(TQ_LOADED0 + (c & 1)));
+        };
+        uint32_t sv[2][32], dv[2][32];
+        if (NG == 1) {  // everything in flight at once; two groups have fewer registers each and work under one another's waits
+#pragma unroll
+          for (int cc = 0; cc < 2; ++cc) {
+            tmem_ld_32x32(my_s + cc * 32, sv[cc]);
+            tmem_ld_32x32(my_dp + cc * 32, dv[cc]);
+          }
+          loaded();
+        }
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc) {
+          if (NG == 2) {
+            tmem_ld_32x32(my_s + cc * 32, sv[cc]);
+            tmem_ld_32x32(my_dp + cc * 32, dv[cc]);
+            if (cc == 0)
+              tmem_ld_wait();
+            else
+              loaded();
+          }
+          const int col0 = half * 64 + cc * 32;
+          float ds[32];
+          if (diag) {  // rows beyond the sequence need no mask: a row of dS reaches its own row of dQ only
+#pragma unroll
+            for (int i2 = 0; i2 < 32; ++i2) {
+              const bool keep = (col0 + i2) <= r;
+              const float p = keep ? fast_exp2(__uint_as_float(sv[cc][i2]) * scale_log2 - lse) : 0.f;
+              ds[i2] = p * (__uint_as_float(dv[cc][i2]) - dl);
+            }
+          } else {
+#pragma unroll
+            for (int i2 = 0; i2 < 32; ++i2) {
+              const float p = fast_exp2(__uint_as_float(sv[cc][i2]) * scale_log2 - lse);
+              ds[i2] = p * (__uint_as_float(dv[cc][i2]) - dl);
+            }
+          }
+          uint32_t packed[16];
+          pack32(ds, packed);
+          tmem_st_32x16(my_s + cc * 16, packed);  // over score columns this thread has already read
+        }
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();  // the lanes' stores are ordered before the one arrival of the warp
+        if (lane == 0) mbar_arrive(bar(TQ_DS_READY0 + (c & 1)));
       }
+      c0 += n_kv;
+      if (ok && (c0 - 1) % NG == g) {  // the group of the last tile stores the item
+        const int qb = u % QB;
+        ok = mbar_wait_warp(bar(TQ_DQ_FULL0 + qb), (u / QB) & 1, abort_flag);
+        if (ok) {
+          tc_fence_after();
+          const long long tok = static_cast<long long>(w.batch) * S + row;
+          store_acc<HD / 2>(t_dq(u) + lane_addr + half * (HD / 2), dQ + tok * lddq + w.head * HD + half * (HD / 2), lddq, scale, S - row);
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(TQ_DQ_EMPTY0 + qb));
+        }
+      }
+      ++u;
     }
     tc_fence_before();
   }
@@ -244,9 +318,9 @@ int launch_dq_tmem(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorM
     if (e != cudaSuccess) return static_cast<int>(e);
     configured = true;
   }
-  const int n_tiles = (S + BLK - 1) / BLK;
-  attn_dq_tmem_kernel<HD><<<dim3(n_tiles * Hq, B, 1), 320, DqTmemSmem<HD>::TOTAL, stream>>>(
-      tq, tk, tv, tdo, lse, delta, static_cast<__nv_bfloat16*>(dq), S, Hq, Hkv, lddq, scale,
+  const int items = (S + BLK - 1) / BLK * Hq * B, sms = sm_count();
+  attn_dq_tmem_kernel<HD><<<items < sms ? items : sms, DqTmemSmem<HD>::THREADS, DqTmemSmem<HD>::TOTAL, stream>>>(
+      tq, tk, tv, tdo, lse, delta, static_cast<__nv_bfloat16*>(dq), B, S, Hq, Hkv, lddq, scale,
       scale * 1.4426950408889634f, status);
   return static_cast<int>(cudaGetLastError());
 }
@@ -556,9 +630,9 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
         const int krow = jt * BLK + r;
         const long long tok = static_cast<long long>(batch) * S + krow;
         if (NG == 1 || g == 0)
-          store_acc<HD / 2>(t_dv + lane_addr + hf * (HD / 2), dV + tok * lddv + kv_head * HD + hf * (HD / 2), 1.f, krow < S);
+          store_acc<HD / 2>(t_dv + lane_addr + hf * (HD / 2), dV + tok * lddv + kv_head * HD + hf * (HD / 2), lddv, 1.f, S - krow);
         if (NG == 1 || g == 1)
-          store_acc<HD / 2>(t_dk + lane_addr + hf * (HD / 2), dK + tok * lddk + kv_head * HD + hf * (HD / 2), scale, krow < S);
+          store_acc<HD / 2>(t_dk + lane_addr + hf * (HD / 2), dK + tok * lddk + kv_head * HD + hf * (HD / 2), lddk, scale, S - krow);
       }
     }
     tc_fence_before();
@@ -606,10 +680,7 @@ int launch_bwd_tmem(const void* dout, const void* q, const void* k, const void* 
   if (!make_attn_tensormap(&tv, v, HD, Hkv, S, B, ldv)) return -4;
   if (!make_attn_tensormap(&tdo, dout, HD, Hq, S, B, static_cast<long long>(Hq) * HD)) return -5;
   cudaGetLastError();
-  const long long warps = static_cast<long long>(B) * S * Hq;
-  if (parts & 1)
-    attn_delta_kernel<HD><<<static_cast<unsigned>((warps * 32 + 255) / 256), 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(o), static_cast<const __nv_bfloat16*>(dout), delta, B, S, Hq);
+  if (parts & 1) launch_delta<HD>(o, dout, delta, B, S, Hq, stream);
   int rc = 0;
   if (parts & 2) rc = launch_dkdv_tmem<HD>(tq, tk, tv, tdo, lse, delta, dk, dv, B, S, Hq, Hkv, lddk, lddv, scale, status, stream);
   if (rc == 0 && (parts & 4)) rc = launch_dq_tmem<HD>(tq, tk, tv, tdo, lse, delta, dq, B, S, Hq, Hkv, lddq, scale, status, stream);

@@ -343,17 +343,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tq, const __grid_consta
           uint32_t ov[32];
           tmem_ld_32x32(o_addr + c * 32, ov);
           tmem_ld_wait();
-          if (row < S) {
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              uint4 u;
-              u.x = pack_bf16(__uint_as_float(ov[g * 8 + 0]) * inv, __uint_as_float(ov[g * 8 + 1]) * inv);
-              u.y = pack_bf16(__uint_as_float(ov[g * 8 + 2]) * inv, __uint_as_float(ov[g * 8 + 3]) * inv);
-              u.z = pack_bf16(__uint_as_float(ov[g * 8 + 4]) * inv, __uint_as_float(ov[g * 8 + 5]) * inv);
-              u.w = pack_bf16(__uint_as_float(ov[g * 8 + 6]) * inv, __uint_as_float(ov[g * 8 + 7]) * inv);
-              reinterpret_cast<uint4*>(dst + c * 32)[g] = u;
-            }
-          }
+          store_rows32(ov, inv, dst + c * 32, ldo, S - row);
         }
         if (row < S) LSE[(static_cast<long long>(batch) * Hq + head) * S + row] = m + log2f(l);
       }

@@ -71,6 +71,8 @@ def attention_bwd(do: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.T
         dq, dk, dv = out
     delta = torch.empty(B, Hq, S, dtype=torch.float32, device=q.device)
     do = do if do.is_contiguous() else do.contiguous()
+    if o.data_ptr() % 16:  # read in 16-byte vectors
+        o = o.clone()
     status = _lib.ptr(_lib.status_word(q.device))
     common = (_lib.ptr(do), _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(o), _lib.ptr(lse), _lib.ptr(delta),
               _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), B, S, Hq, Hkv, D,
