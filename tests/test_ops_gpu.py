@@ -362,3 +362,30 @@ def test_outer_step_reads_and_writes_the_parameters_in_place(dtype, momentum, ne
                 assert ((got - bufs[i]).abs() <= 2.0**-22 * (bufs[i].abs() + g.abs())).all()
                 bufs[i] = got.clone()
             old[i] = p.detach().clone()
+
+
+@pytest.mark.parametrize("V", [8, 248, 256, 264, 2056, 32768, 32776, 65536, 65544, 128256, 262144, 262152])
+def test_cross_entropy_around_the_sizes_of_a_row_in_registers(V):
+    """One warp, whole blocks, clusters of two to eight CTAs and the two-pass kernel beyond them; targets at both ends of the
+    row and around the borders of the parts, logits of -inf (also a whole first vector of them) and an ignored row."""
+    from torchft_b200.ops.functional import cross_entropy
+
+    torch.manual_seed(V)
+    marks = sorted({t for t in (0, 7, 8, 255, V // 8, V // 4 - 1, V // 4, V // 2 - 1, V // 2, V // 2 + 3, V - 8, V - 1) if 0 <= t < V})
+    targets = torch.tensor(marks + [-100], device=DEV)
+    logits = bf16(len(targets), V, scale=3.0)
+    kept = torch.zeros(len(targets), V, dtype=torch.bool, device=DEV)
+    kept[torch.arange(len(marks)), targets[:-1]] = True
+    logits[torch.rand(len(targets), V, device=DEV).lt(0.1) & ~kept] = float("-inf")
+    if V > 8 and 0 not in marks[-3:]:
+        logits[-3, :8] = float("-inf")
+    x = logits.double().requires_grad_()
+    ref = torch.nn.functional.cross_entropy(x, targets, ignore_index=-100)
+    ref.backward()
+    work = logits.clone().requires_grad_()
+    loss = cross_entropy(work, targets, ignore_index=-100)
+    loss.backward()
+    # fp32 sums of exponentials good to 2e-6 each, and one rounding to bf16 of every gradient
+    assert abs(loss.item() - ref.item()) < 2e-5 * max(1.0, abs(ref.item()))
+    assert ((work.grad.double() - x.grad).abs() <= 2.0**-8 * x.grad.abs() + 4e-6 / len(marks)).all()
+    assert (work.grad[-1] == 0).all()

@@ -69,68 +69,173 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __
 }
 
 // ------------------------------------------------------------------ cross entropy
-// One block per row of logits [rows, V] (bf16).  Pass 1: online max / sum-exp.
-// Pass 2 (in place): logits <- (softmax - onehot) * grad_scale.  loss[row] = lse - z_target.
-// Rows whose target is ignore_index produce zero loss and zero gradient.
-__global__ void xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets,
-                            float* __restrict__ loss, int V, int ld, float grad_scale, long long ignore_index) {
-  __shared__ float red_m[32], red_s[32];
+// logits <- (softmax - onehot) * grad_scale, loss[row] = lse - z_target.  Rows whose target is ignore_index produce
+// zero loss and zero gradient.
+//
+// Two kernels.  Rows of up to 32768 columns stay in the registers of one block between the two passes, eight 16-byte
+// vectors a thread (xent_row_kernel).  Longer rows are read twice, the second time partly from L2 (xent_kernel): holding
+// them in the registers of a cluster of CTAs reads memory once but costs a cluster barrier a row, and took 311 to 430 us
+// where the two passes take 205 (2048 x 128256).
+constexpr int XENT_VECS = 8;
+constexpr int XENT_THREADS = 512;
+constexpr int XENT_ROOM = XENT_THREADS * XENT_VECS;  // vectors of a row that one block takes
+
+struct MaxSum {
+  float m, s;  // maximum and sum of exp(x - m); an empty or all -inf part is (-inf, 0)
+};
+__device__ __forceinline__ MaxSum combine(MaxSum a, MaxSum b) {
+  MaxSum r;
+  r.m = fmaxf(a.m, b.m);
+  r.s = (a.m == -INFINITY ? 0.f : a.s * __expf(a.m - r.m)) + (b.m == -INFINITY ? 0.f : b.s * __expf(b.m - r.m));
+  return r;
+}
+__device__ __forceinline__ MaxSum warp_combine(MaxSum v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    MaxSum w;
+    w.m = __shfl_xor_sync(0xffffffffu, v.m, o);
+    w.s = __shfl_xor_sync(0xffffffffu, v.s, o);
+    v = combine(v, w);
+  }
+  return v;
+}
+
+// The gradient of eight logits f of which element `here` (if below 8) is the target.  exp(f - lse) as one multiply-add and one
+// exp2; the target's own value, from which 1 is taken, without the rounding of lse * log2(e).
+constexpr float kLog2e = 1.4426950408889634f;
+__device__ __forceinline__ uint4 xent_grad(const uint4& u, float lse, float scale, unsigned here, float* loss) {
+  float f[8];
+  ew_unpack8(u, f);
+  float hot = 0.f;
+  if (here < 8u) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (here == j) hot = f[j];
+    *loss = lse - hot;
+    hot = (__expf(hot - lse) - 1.f) * scale;
+  }
+  const float c = lse * kLog2e;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) f[j] = exp2f(fmaf(f[j], kLog2e, -c)) * scale;
+  if (here < 8u) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (here == j) f[j] = hot;
+  }
+  return ew_pack8(f);
+}
+
+// One block per row, as few threads as hold it: short rows then share an SM with more of their kind.  Bound by the launch
+// below a few thousand rows; 14.7 us for 26.6 with two passes at 2048 x 4096, 33.8 for 63.8 at 4096 x 8192, 7.9 for 12.8 at
+// 1024 x 1000, 265 for 281 at 8192 x 32000.
+__global__ void __launch_bounds__(XENT_THREADS, 2)
+xent_row_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets, float* __restrict__ loss, int V,
+                int ld, float grad_scale, long long ignore_index) {
+  __shared__ MaxSum part[32];  // one per warp
   const size_t row = blockIdx.x;
-  __nv_bfloat16* z = logits + row * ld;
+  const int n = V / 8, step = blockDim.x;
+  uint4* z = reinterpret_cast<uint4*>(logits + row * ld) + threadIdx.x;
   const long long tgt = targets[row];
-  const int nvec = V / 8;
-  float m = -INFINITY, s = 0.f;
-  for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
+  uint4 v[XENT_VECS];
+#pragma unroll
+  for (int k = 0; k < XENT_VECS; ++k)
+    v[k] = static_cast<int>(threadIdx.x) + k * step < n ? z[k * step] : make_uint4(0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u);  // -inf
+  MaxSum r = {-INFINITY, 0.f};
+#pragma unroll
+  for (int k = 0; k < XENT_VECS; ++k) {
     float f[8];
-    ew_unpack8(reinterpret_cast<const uint4*>(z)[i], f);
-    float lm = f[0];
+    ew_unpack8(v[k], f);
 #pragma unroll
-    for (int j = 1; j < 8; ++j) lm = fmaxf(lm, f[j]);
-    const float nm = fmaxf(m, lm);
-    float ls = 0.f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) ls += __expf(f[j] - nm);
-    s = s * __expf(m - nm) + ls;
-    m = nm;
+    for (int j = 0; j < 8; ++j) r.m = fmaxf(r.m, f[j]);
   }
-  // combine (m, s) pairs across the block
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float base = r.m == -INFINITY ? 0.f : r.m;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float om = __shfl_xor_sync(0xffffffffu, m, o);
-    const float os = __shfl_xor_sync(0xffffffffu, s, o);
-    const float nm = fmaxf(m, om);
-    s = (m == -INFINITY ? 0.f : s * __expf(m - nm)) + (om == -INFINITY ? 0.f : os * __expf(om - nm));
-    m = nm;
-  }
-  if (lane == 0) { red_m[warp] = m; red_s[warp] = s; }
-  __syncthreads();
-  const int nw = blockDim.x >> 5;
-  m = lane < nw ? red_m[lane] : -INFINITY;
-  s = lane < nw ? red_s[lane] : 0.f;
+  for (int k = 0; k < XENT_VECS; ++k) {
+    float f[8];
+    ew_unpack8(v[k], f);
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float om = __shfl_xor_sync(0xffffffffu, m, o);
-    const float os = __shfl_xor_sync(0xffffffffu, s, o);
-    const float nm = fmaxf(m, om);
-    s = (m == -INFINITY ? 0.f : s * __expf(m - nm)) + (om == -INFINITY ? 0.f : os * __expf(om - nm));
-    m = nm;
+    for (int j = 0; j < 8; ++j) r.s += __expf(f[j] - base);
   }
-  const float lse = m + __logf(s);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  r = warp_combine(r);
+  if (warps > 1) {
+    if (lane == 0) part[warp] = r;
+    __syncthreads();
+    r = warp_combine(lane < warps ? part[lane] : MaxSum{-INFINITY, 0.f});
+  }
+  const float lse = r.m + __logf(r.s);
   const bool ignored = tgt == ignore_index || tgt < 0 || tgt >= V;
-  if (threadIdx.x == 0) loss[row] = ignored ? 0.f : lse - __bfloat162float(z[tgt]);
-  __syncthreads();  // the target logit is read before it is overwritten below
+  if (ignored && threadIdx.x == 0) loss[row] = 0.f;
   const float scale = ignored ? 0.f : grad_scale;
-  for (int i = threadIdx.x; i < nvec; i += blockDim.x) {
-    float f[8];
-    ew_unpack8(reinterpret_cast<const uint4*>(z)[i], f);
+  // place of the target among this thread's vectors: element hot % 8 of vector hot / 8 counted from its first
+  const int hot = ignored ? -1 : static_cast<int>(tgt) - static_cast<int>(threadIdx.x) * 8;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float p = __expf(f[j] - lse);
-      if (i * 8 + j == tgt) p -= 1.f;
-      f[j] = p * scale;
+  for (int k = 0; k < XENT_VECS; ++k, z += step) {
+    if (static_cast<int>(threadIdx.x) + k * step >= n) break;
+    *z = xent_grad(v[k], lse, scale, static_cast<unsigned>(hot - k * step * 8), loss + row);
+  }
+}
+
+// Pass 1: online maximum and sum of exponentials.  Pass 2 (in place): the gradient.  Two vectors a thread and round in flight,
+// two blocks of 1024 per SM: 205 us at 2048 x 128256 (158 for one read and one write at the copy bandwidth), 241 with one.
+// Four vectors and half the threads: 215; one block per SM: 214.
+constexpr int XENT_LONG_THREADS = 1024;
+constexpr int XENT_LONG_VECS = 2;
+__global__ void __launch_bounds__(XENT_LONG_THREADS, 2)
+xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets, float* __restrict__ loss, int V, int ld,
+            float grad_scale, long long ignore_index) {
+  __shared__ MaxSum part[32];
+  constexpr int U = XENT_LONG_VECS, STEP = XENT_LONG_THREADS;
+  const size_t row = blockIdx.x;
+  const int n = V / 8;
+  uint4* z = reinterpret_cast<uint4*>(logits + row * ld);
+  const long long tgt = targets[row];
+  MaxSum r = {-INFINITY, 0.f};
+  for (int i0 = threadIdx.x; i0 < n; i0 += U * STEP) {
+    uint4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      v[u] = i0 + u * STEP < n ? z[i0 + u * STEP] : make_uint4(0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u);  // -inf
+    float m = r.m;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float f[8];
+      ew_unpack8(v[u], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) m = fmaxf(m, f[j]);
     }
-    reinterpret_cast<uint4*>(z)[i] = ew_pack8(f);
+    if (m == -INFINITY) continue;  // nothing but -inf so far
+    float s = 0.f;
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      float f[8];
+      ew_unpack8(v[u], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s += __expf(f[j] - m);
+    }
+    r.s = r.s * __expf(r.m - m) + s;
+    r.m = m;
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  r = warp_combine(r);
+  if (lane == 0) part[warp] = r;
+  __syncthreads();
+  r = warp_combine(part[lane]);
+  const float lse = r.m + __logf(r.s);
+  const bool ignored = tgt == ignore_index || tgt < 0 || tgt >= V;
+  if (ignored && threadIdx.x == 0) loss[row] = 0.f;
+  const float scale = ignored ? 0.f : grad_scale;
+  const int hot = ignored ? -1 : static_cast<int>(tgt);
+  for (int i0 = threadIdx.x; i0 < n; i0 += U * STEP) {
+    uint4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (i0 + u * STEP < n) v[u] = z[i0 + u * STEP];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u * STEP;
+      if (i < n) z[i] = xent_grad(v[u], lse, scale, static_cast<unsigned>(hot - i * 8), loss + row);
+    }
   }
 }
 
@@ -429,8 +534,13 @@ TFT_API int tft_swiglu_bwd(const void* gu, const void* dout, void* dgu, long lon
 TFT_API int tft_xent(void* logits, const long long* targets, float* loss, int rows, int V, int ld,
                      float grad_scale, long long ignore_index, cudaStream_t stream) {
   if (V % 8 || ld % 8) return static_cast<int>(cudaErrorInvalidValue);
-  xent_kernel<<<rows, 1024, 0, stream>>>(static_cast<__nv_bfloat16*>(logits), targets, loss, V, ld, grad_scale,
-                                         ignore_index);
+  auto* z = static_cast<__nv_bfloat16*>(logits);
+  const int vecs = V / 8;
+  if (vecs <= XENT_ROOM)
+    xent_row_kernel<<<rows, (vecs + 32 * XENT_VECS - 1) / (32 * XENT_VECS) * 32, 0, stream>>>(z, targets, loss, V, ld, grad_scale,
+                                                                                             ignore_index);
+  else
+    xent_kernel<<<rows, XENT_LONG_THREADS, 0, stream>>>(z, targets, loss, V, ld, grad_scale, ignore_index);
   return static_cast<int>(cudaGetLastError());
 }
 
