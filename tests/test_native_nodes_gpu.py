@@ -1,0 +1,129 @@
+"""The native autograd nodes give the values of the Python nodes, and leave to those every call that is not plain."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+DEV = "cuda"
+
+
+def leaf(*shape, scale=1.0):
+    return (torch.randn(*shape, device=DEV) * scale).to(torch.bfloat16).requires_grad_()
+
+
+def both(native, python, inputs):
+    """Outputs and gradients of the two routes for the same inputs and upstream gradients."""
+    results = []
+    for fn in (native, python):
+        outs = fn(*inputs)
+        outs = outs if isinstance(outs, tuple) else (outs,)
+        torch.manual_seed(1)
+        ups = [torch.randn_like(o) for o in outs]
+        grads = torch.autograd.grad(outs, inputs, ups)
+        results.append([o.detach() for o in outs] + list(grads))
+    return results
+
+
+CASES = {
+    "linear": lambda F, A: (F.linear, F._Linear.apply, [leaf(3, 50, 72), leaf(40, 72)]),
+    "rmsnorm": lambda F, A: (F.rmsnorm, lambda x, w: F._RMSNorm.apply(x, w, 1e-5), [leaf(5, 256), leaf(256)]),
+    "add_rmsnorm": lambda F, A: (F.add_rmsnorm, lambda x, r, w: F._AddRMSNorm.apply(x, r, w, 1e-5),
+                                 [leaf(2, 9, 768), leaf(2, 9, 768), leaf(768)]),
+    "swiglu": lambda F, A: (F.swiglu, F._SwiGLU.apply, [leaf(7, 2 * 24)]),
+    "attention": lambda F, A: (A.attention, lambda q, k, v: A._Attention.apply(q, k, v, None),
+                               [leaf(2, 70, 4, 64), leaf(2, 70, 2, 64), leaf(2, 70, 2, 64)]),
+}
+
+
+@pytest.mark.parametrize("name", CASES)
+def test_native_and_python_nodes_agree(name):
+    """Same kernels on the same operands: equal bit for bit."""
+    from torchft_b200.ops import attention as A
+    from torchft_b200.ops import functional as F
+
+    torch.manual_seed(0)
+    native, python, inputs = CASES[name](F, A)
+    out = native(*inputs)
+    node = (out[0] if isinstance(out, tuple) else out).grad_fn
+    assert not isinstance(node, torch.autograd.function.BackwardCFunction)  # the base of every Python node
+    for a, b in zip(*both(native, python, inputs)):
+        assert torch.equal(a, b)
+
+
+def test_calls_that_stay_with_the_python_nodes():
+    from torchft_b200.ops import _native
+    from torchft_b200.ops import functional as F
+
+    m = _native.module()
+    x, w = leaf(16, 64), leaf(32, 64)
+    assert m.linear(x, w) is not None
+    wide = torch.zeros(16, 128, device=DEV, dtype=torch.bfloat16)
+    odd = torch.zeros(16 * 64 + 1, device=DEV, dtype=torch.bfloat16)[1:].view(16, 64)
+    marked = leaf(32, 64)
+    marked.main_grad = torch.zeros_like(marked)
+    for a, b in ((wide[:, :64], w), (odd, w), (x.float(), w), (x.cpu(), w), (x, marked), (leaf(16, 60), leaf(32, 60)), (x[:0], w)):
+        assert m.linear(a, b) is None
+    assert m.rmsnorm(leaf(4, 264), leaf(264), 1e-5) is None  # a width that the kernel has no split for
+    assert m.swiglu(leaf(4, 24)) is None
+    torch.manual_seed(0)
+    strided = torch.randn(16, 128, device=DEV).to(torch.bfloat16)[:, ::2]
+    assert m.linear(strided, w) is None
+    with torch.no_grad():  # inference is plain
+        assert m.linear(x, w).grad_fn is None
+
+    seen = []
+
+    def transformed(x_):
+        seen.append(m.linear(x_, w.detach()) is None and m.linear(x.detach(), w.detach()) is None)
+        return x_.sum()
+
+    torch.func.grad(transformed)(x.detach())
+    assert seen == [True]
+    with torch.autograd.forward_ad.dual_level():
+        dual = torch.autograd.forward_ad.make_dual(x.detach(), torch.ones_like(x))
+        assert m.linear(dual, w) is None
+    with pytest.raises(F._lib.KernelError):
+        F.linear(leaf(16, 60), leaf(32, 60))
+
+
+def test_saved_tensor_hooks_and_late_gradient_buffers():
+    from torchft_b200.ops import functional as F
+
+    torch.manual_seed(0)
+    x, w = leaf(16, 64), leaf(32, 64)
+    packed = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (packed.append(t.shape), t.cpu())[1], lambda t: t.to(DEV)):
+        y = F.linear(x, w)
+    dy = torch.randn_like(y)
+    dx, dw = torch.autograd.grad(y, (x, w), dy)
+    assert torch.Size((16, 64)) in packed and torch.Size((32, 64)) in packed
+    ref = F._Linear.apply(x, w)
+    rx, rw = torch.autograd.grad(ref, (x, w), dy)
+    assert torch.equal(dx, rx) and torch.equal(dw, rw)
+
+    # buffers that an engine gives to the weights between forward and backward receive the gradients
+    n = leaf(256)
+    x, w = leaf(16, 256), leaf(32, 256)
+    y = F.linear(F.rmsnorm(x, n), w)
+    for p in (w, n):
+        p.main_grad = torch.full_like(p, float("nan"))
+    y.backward(dy)
+    assert w.grad is None and n.grad is None
+    assert torch.isfinite(w.main_grad).all() and w.main_grad_initialized
+    want = dy.float().t() @ F.rmsnorm(x, n.detach().clone()).detach().float()
+    assert (w.main_grad.float() - want).norm() < 8e-3 * want.norm()  # one rounding of the sum to bf16
+
+
+def test_cross_entropy_matches_the_python_node():
+    from torchft_b200.ops import functional as F
+
+    torch.manual_seed(0)
+    logits, targets = torch.randn(33, 1000, device=DEV).to(torch.bfloat16), torch.randint(1000, (33,), device=DEV)
+    got = []
+    for fn in (F.cross_entropy, lambda z, t: F._CrossEntropy.apply(z, t, None)):
+        z = logits.clone().requires_grad_()
+        loss = fn(z, targets)
+        loss.backward()
+        got.append((loss.detach(), z.grad))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])

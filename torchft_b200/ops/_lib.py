@@ -10,7 +10,7 @@ from __future__ import annotations
 import ctypes
 import threading
 from ctypes import c_float, c_int, c_int64, c_void_p
-from typing import Optional
+from typing import Callable, List, Optional
 
 import torch
 
@@ -77,8 +77,10 @@ def available() -> bool:
 
 
 def stream_ptr(stream: Optional[torch.cuda.Stream] = None) -> int:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    if stream is not None:
+        return stream.cuda_stream
+    # the handle alone: the Stream object around it costs more than the launch
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def ptr(t: Optional[torch.Tensor]) -> int:
@@ -100,8 +102,16 @@ def count_launch(n: int = 1) -> None:
     _launches += n
 
 
+_counters: List[Callable[[], int]] = []
+
+
+def add_launch_counter(counter: Callable[[], int]) -> None:
+    """Registers the count of a native module that launches kernels by itself."""
+    _counters.append(counter)
+
+
 def launches() -> int:
-    return _launches
+    return _launches + sum(counter() for counter in _counters)
 
 
 _status: dict = {}

@@ -11,8 +11,8 @@ from typing import Optional, Tuple
 
 import torch
 
-from . import _lib
-from .gemm import gemm
+from . import _lib, _native
+from .gemm import DEFAULT_IMPL, gemm
 
 
 def _check_bf16(*tensors: torch.Tensor) -> None:
@@ -67,28 +67,34 @@ class _Linear(torch.autograd.Function):
             dx = gemm(dy2, w, b_kmajor=False).view(ctx.x_shape)  # dY [M,N] @ W [N,K]
         dw = None
         if ctx.needs_input_grad[1]:
-            weight = ctx.weight
-            main_grad = getattr(weight, "main_grad", None)
-            rs_comm = getattr(weight, "rs_comm", None)
-            if main_grad is not None and rs_comm is not None:
-                # rows of the weight are sharded over the GPUs of the group: the GEMM's epilogue sends
-                # every tile to its owner, and only this rank's rows of the summed gradient are written
-                acc = bool(getattr(weight, "main_grad_initialized", False))
-                rows = weight.shape[0] // rs_comm.world
-                own = main_grad[rs_comm.rank * rows : (rs_comm.rank + 1) * rows]
-                rs_comm.wgrad_reduce_scatter(dy2, x2, own, accumulate=acc)
-                weight.main_grad_initialized = True
-            elif main_grad is not None:
-                acc = bool(getattr(weight, "main_grad_initialized", False))
-                gemm(dy2, x2, main_grad, a_kmajor=False, b_kmajor=False, accumulate=acc)  # dY^T @ X
-                weight.main_grad_initialized = True
-            else:
-                dw = gemm(dy2, x2, a_kmajor=False, b_kmajor=False)
+            dw = _weight_gradient(ctx.weight, dy2, x2)
         return dx, dw
 
 
+def _weight_gradient(weight: torch.Tensor, dy2: torch.Tensor, x2: torch.Tensor) -> Optional[torch.Tensor]:
+    """``dY^T @ X`` as a new tensor, or ``None`` after it went where the weight's attributes say."""
+    main_grad = getattr(weight, "main_grad", None)
+    rs_comm = getattr(weight, "rs_comm", None)
+    if main_grad is not None and rs_comm is not None:
+        # rows of the weight are sharded over the GPUs of the group: the GEMM's epilogue sends
+        # every tile to its owner, and only this rank's rows of the summed gradient are written
+        acc = bool(getattr(weight, "main_grad_initialized", False))
+        rows = weight.shape[0] // rs_comm.world
+        own = main_grad[rs_comm.rank * rows : (rs_comm.rank + 1) * rows]
+        rs_comm.wgrad_reduce_scatter(dy2, x2, own, accumulate=acc)
+        weight.main_grad_initialized = True
+        return None
+    if main_grad is not None:
+        acc = bool(getattr(weight, "main_grad_initialized", False))
+        gemm(dy2, x2, main_grad, a_kmajor=False, b_kmajor=False, accumulate=acc)  # dY^T @ X
+        weight.main_grad_initialized = True
+        return None
+    return gemm(dy2, x2, a_kmajor=False, b_kmajor=False)
+
+
 def linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
-    return _Linear.apply(x, w)
+    y = _native.module().linear(x, w) if DEFAULT_IMPL == "pair" else None
+    return _Linear.apply(x, w) if y is None else y
 
 
 # ------------------------------------------------------------------ RMSNorm
@@ -185,11 +191,13 @@ class _AddRMSNorm(torch.autograd.Function):
 
 
 def rmsnorm(x: torch.Tensor, w: torch.Tensor, eps: float = 1e-5) -> torch.Tensor:
-    return _RMSNorm.apply(x, w, eps)
+    y = _native.module().rmsnorm(x, w, eps)
+    return _RMSNorm.apply(x, w, eps) if y is None else y
 
 
 def add_rmsnorm(x: torch.Tensor, res: torch.Tensor, w: torch.Tensor, eps: float = 1e-5) -> Tuple[torch.Tensor, torch.Tensor]:
-    return _AddRMSNorm.apply(x, res, w, eps)
+    out = _native.module().add_rmsnorm(x, res, w, eps)
+    return _AddRMSNorm.apply(x, res, w, eps) if out is None else out
 
 
 # ------------------------------------------------------------------ RoPE
@@ -249,7 +257,8 @@ class _SwiGLU(torch.autograd.Function):
 
 def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
     """``silu(gate) * up`` for ``gate_up[..., :F] = gate`` and ``gate_up[..., F:] = up``."""
-    return _SwiGLU.apply(gate_up)
+    out = _native.module().swiglu(gate_up)
+    return _SwiGLU.apply(gate_up) if out is None else out
 
 
 # ------------------------------------------------------------------ cross entropy
@@ -286,7 +295,8 @@ class _CrossEntropy(torch.autograd.Function):
 def cross_entropy(logits: torch.Tensor, targets: torch.Tensor, ignore_index: Optional[int] = None) -> torch.Tensor:
     """Mean cross entropy.  ``logits`` is consumed: after the call it holds the gradient
     (valid for ``loss.backward()`` with unit upstream gradient)."""
-    return _CrossEntropy.apply(logits, targets, ignore_index)
+    loss = _native.module().cross_entropy(logits, targets) if ignore_index is None else None
+    return _CrossEntropy.apply(logits, targets, ignore_index) if loss is None else loss
 
 
 # ------------------------------------------------------------------ embedding

@@ -1,10 +1,12 @@
 """In-tree native builds.
 
-Two artefacts are produced next to the Python sources:
+Three artefacts are produced next to the Python sources:
 
 * ``torchft_b200/lib/libtft_kernels.so`` -- every ``.cu`` file under ``csrc/kernels``
   compiled with nvcc for ``sm_100a`` and exported through a plain C ABI (loaded with
   ctypes, no link-time dependency on torch or libcuda).
+* ``torchft_b200/_autograd.*.so`` -- native autograd nodes over the kernels (``csrc/host``), the one
+  artefact compiled against torch's headers.
 * ``torchft_b200/_control.*.so`` -- the C++ control plane (lighthouse, manager server and
   client) as a pybind11 extension module, plus the ``tft_lighthouse`` executable.
 
@@ -24,6 +26,7 @@ from typing import List
 PKG = Path(__file__).resolve().parent.parent
 KERNEL_SRC = PKG / "csrc" / "kernels"
 CONTROL_SRC = PKG / "csrc" / "control"
+HOST_SRC = PKG / "csrc" / "host"
 LIB_DIR = PKG / "lib"
 OBJ_DIR = PKG / "lib" / "obj"
 
@@ -58,6 +61,11 @@ def kernels_lib_path() -> Path:
 def control_module_path() -> Path:
     suffix = sysconfig.get_config_var("EXT_SUFFIX") or ".so"
     return PKG / f"_control{suffix}"
+
+
+def autograd_module_path() -> Path:
+    suffix = sysconfig.get_config_var("EXT_SUFFIX") or ".so"
+    return PKG / f"_autograd{suffix}"
 
 
 def lighthouse_bin_path() -> Path:
@@ -99,6 +107,36 @@ def build_kernels(force: bool = False, verbose: bool = False) -> Path:
     return out
 
 
+def _host_cxx() -> str:
+    # Prefer the distribution compiler: it links libstdc++ dynamically, so a module
+    # shares one C++ runtime with torch.
+    return os.environ.get("TFT_CXX") or ("/usr/bin/g++" if Path("/usr/bin/g++").exists() else os.environ.get("CXX", "g++"))
+
+
+def build_autograd(force: bool = False) -> Path:
+    """Builds the native autograd nodes against the installed torch."""
+    import torch
+
+    src = HOST_SRC / "autograd.cc"
+    out = autograd_module_path()
+    torch_dir = Path(torch.__file__).parent
+    # rebuilt for another torch as well: the module follows its C++ interface
+    newest = max(_newest([src]), (torch_dir / "version.py").stat().st_mtime)
+    if not force and out.exists() and out.stat().st_mtime >= newest:
+        return out
+    cuda_home = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
+    cmd = [_host_cxx(), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_EXTENSION_NAME=_autograd",
+           "-DTORCH_API_INCLUDE_EXTENSION_H", "-I", str(torch_dir / "include"),
+           "-I", str(torch_dir / "include" / "torch" / "csrc" / "api" / "include"), "-I", str(cuda_home / "include"),
+           "-I", sysconfig.get_paths()["include"], str(src), "-o", str(out), "-L", str(torch_dir / "lib"),
+           "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"autograd build failed:\n{res.stdout}\n{res.stderr}")
+    return out
+
+
 def build_control(force: bool = False) -> Path:
     """Builds the pybind11 control-plane module and the standalone lighthouse binary."""
     import pybind11
@@ -108,10 +146,9 @@ def build_control(force: bool = False) -> Path:
     headers = sorted(CONTROL_SRC.glob("*.h"))
     out = control_module_path()
     newest = max(_newest(sources), _newest(headers))
-    # Prefer the distribution compiler: it links libstdc++ dynamically, so the module
-    # shares one C++ runtime with torch.  -Bsymbolic keeps a statically linked runtime
-    # (other toolchains) from being half-interposed by the process-wide one.
-    cxx = os.environ.get("TFT_CXX") or ("/usr/bin/g++" if Path("/usr/bin/g++").exists() else os.environ.get("CXX", "g++"))
+    # -Bsymbolic keeps a statically linked runtime (other toolchains) from being
+    # half-interposed by the process-wide one.
+    cxx = _host_cxx()
     common = ["-O2", "-std=c++17", "-fPIC", "-pthread", "-Wall", "-Wno-unused-function", "-Wl,-Bsymbolic"]
     if force or not out.exists() or out.stat().st_mtime < newest:
         py_inc = sysconfig.get_paths()["include"]
@@ -134,8 +171,9 @@ def build_control(force: bool = False) -> Path:
 def build_all(force: bool = False, verbose: bool = False) -> None:
     build_control(force=force)
     build_kernels(force=force, verbose=verbose)
+    build_autograd(force=force)
 
 
 if __name__ == "__main__":
     build_all(force="--force" in sys.argv, verbose="-v" in sys.argv)
-    print("built", kernels_lib_path(), control_module_path())
+    print("built", kernels_lib_path(), control_module_path(), autograd_module_path())
