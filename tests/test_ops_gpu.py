@@ -389,3 +389,31 @@ def test_cross_entropy_around_the_sizes_of_a_row_in_registers(V):
     assert abs(loss.item() - ref.item()) < 2e-5 * max(1.0, abs(ref.item()))
     assert ((work.grad.double() - x.grad).abs() <= 2.0**-8 * x.grad.abs() + 4e-6 / len(marks)).all()
     assert (work.grad[-1] == 0).all()
+
+
+def test_adamw_of_many_tensors_equals_one_at_a_time():
+    """Sizes around a vector and a block's chunk, an empty tensor, more tensors than one table holds: bit for bit the same."""
+    from torchft_b200.ops.functional import adamw_multi_, adamw_step_
+
+    torch.manual_seed(0)
+    sizes = [1, 7, 8, 9, 4095, 4096, 4097, 4104, 3 * 4096 + 5, 0] + [5 + i for i in range(90)]
+    kw = dict(lr=3e-4, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, step=3, grad_scale=0.5)
+    ps, gs = [bf16(n) for n in sizes], [bf16(n) for n in sizes]
+    ms, vs = [torch.randn(n, device=DEV) for n in sizes], [torch.rand(n, device=DEV) for n in sizes]
+    single = [[t.clone() for t in ts] for ts in (ps, ms, vs)]
+    adamw_multi_(ps, gs, ms, vs, **kw)
+    for p, g, m, v in zip(single[0], gs, *single[1:]):
+        adamw_step_(p, g, m, v, **kw)
+    for got, want in zip((ps, ms, vs), single):
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
+    # and against the formula in 64 bits: fp32 moments to a few roundings, the parameter to one rounding of bf16
+    n = 8 * 1000 + 5
+    p, g, m, v = bf16(n), bf16(n), torch.randn(n, device=DEV), torch.rand(n, device=DEV)
+    gd = g.double() * 0.5
+    md, vd = 0.9 * m.double() + 0.1 * gd, 0.95 * v.double() + 0.05 * gd * gd
+    want = p.double() * (1 - 3e-4 * 0.1) - 3e-4 * (md / (1 - 0.9**3)) / ((vd / (1 - 0.95**3)).sqrt() + 1e-8)
+    m_old = m.clone()
+    adamw_multi_([p], [g], [m], [v], **kw)
+    # (1 - beta in fp32 is good to 2.4e-7)
+    assert ((m - md).abs() <= 2.0**-21 * (m_old.abs() + gd.abs())).all() and ((v - vd).abs() <= 2.0**-21 * vd).all()
+    assert ((p - want).abs() <= 2.0**-8 * want.abs() + 1e-6).all()

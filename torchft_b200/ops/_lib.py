@@ -36,6 +36,7 @@ _PROTOTYPES = {
     "tft_embedding_fwd": [P, P, P, L, I, P],
     "tft_embedding_bwd": [P, P, P, L, I, P],
     "tft_adamw": [P, P, P, P, L, F, F, F, F, F, I, F, P],
+    "tft_adamw_multi": [P, P, P, P, P, I, F, F, F, F, F, I, F, P],
     "tft_pseudograd": [P, P, P, I, P, P, I, P],
     "tft_nesterov_outer": [P, P, P, I, P, P, P, F, F, I, I, I, P],
     "tft_attn_fwd": [P, P, P, P, P, I, I, I, I, I, I, I, I, F, P, P],

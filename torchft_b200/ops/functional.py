@@ -7,7 +7,8 @@ implementation of the same operation.
 
 from __future__ import annotations
 
-from typing import Optional, Tuple
+import ctypes
+from typing import Optional, Sequence, Tuple
 
 import torch
 
@@ -355,3 +356,24 @@ def adamw_step_(p: torch.Tensor, g: torch.Tensor, m: torch.Tensor, v: torch.Tens
                                 weight_decay, step, grad_scale, _lib.stream_ptr())
     _lib.check(code, "tft_adamw")
     _lib.count_launch()
+
+
+def adamw_multi_(ps: Sequence[torch.Tensor], gs: Sequence[torch.Tensor], ms: Sequence[torch.Tensor], vs: Sequence[torch.Tensor],
+                 *, lr: float, beta1: float, beta2: float, eps: float, weight_decay: float, step: int,
+                 grad_scale: float = 1.0) -> None:
+    """``adamw_step_`` of many buffers in one launch (as many as one table of addresses holds)."""
+    n = len(ps)
+    sizes = []
+    for p, g, m, v in zip(ps, gs, ms, vs):
+        assert p.dtype == torch.bfloat16 and g.dtype == torch.bfloat16 and m.dtype == torch.float32 and v.dtype == torch.float32
+        assert p.is_contiguous() and g.is_contiguous() and m.is_contiguous() and v.is_contiguous()
+        size = p.numel()
+        assert g.numel() == size and m.numel() == size and v.numel() == size
+        sizes.append(size)
+    pointers = ctypes.c_void_p * n
+    code = _lib.lib().tft_adamw_multi(
+        pointers(*[t.data_ptr() for t in ps]), pointers(*[t.data_ptr() for t in gs]), pointers(*[t.data_ptr() for t in ms]),
+        pointers(*[t.data_ptr() for t in vs]), (ctypes.c_int64 * n)(*sizes), n, lr, beta1, beta2, eps, weight_decay, step,
+        grad_scale, _lib.stream_ptr())
+    _lib.check(max(-code, 0), "tft_adamw")
+    _lib.count_launch(code)
