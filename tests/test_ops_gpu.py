@@ -417,3 +417,37 @@ def test_adamw_of_many_tensors_equals_one_at_a_time():
     # (1 - beta in fp32 is good to 2.4e-7)
     assert ((m - md).abs() <= 2.0**-21 * (m_old.abs() + gd.abs())).all() and ((v - vd).abs() <= 2.0**-21 * vd).all()
     assert ((p - want).abs() <= 2.0**-8 * want.abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("a_k,b_k", [(True, True), (True, False), (False, False)])
+@pytest.mark.parametrize("shape", [(1, 8, 2048), (256, 256, 2045 * 8), (257, 264, 2112), (1013, 2048, 5464), (300, 4600, 4104), (9471, 8, 2056)])
+def test_gemm_with_a_divided_contraction(shape, a_k, b_k):
+    """One tile in sixteen parts, ragged tiles, a last part shorter than the others, a contraction that ends inside a k-block,
+    and 36 and 37 tiles, the most that are divided (on 74 CTA pairs)."""
+    from torchft_b200.ops import _lib
+    from torchft_b200.ops.gemm import gemm
+
+    M, N, K = shape
+    if not a_k:
+        M += -M % 8  # the row stride of the transposed operand
+    torch.manual_seed(K)
+    a = bf16(M, K) if a_k else bf16(K, M)
+    b = bf16(N, K) if b_k else bf16(K, N)
+    ref = (a.double() if a_k else a.double().t()) @ (b.double().t() if b_k else b.double())
+    kw = dict(a_kmajor=a_k, b_kmajor=b_k)
+    assert _lib.lib().tft_gemm2_workspace(M, N, K) > 0
+    out32 = gemm(a, b, out_dtype=torch.float32, **kw)
+    whole = gemm(a, b, out_dtype=torch.float32, impl="single", **kw)
+    # The tensor core drops what falls below the last bit of the running fp32 sum, up to 2^-23 of it in each of K / 16 steps,
+    # so shorter parts can only come closer to the exact sum (a tenth allowed for the draw).
+    assert norm_err(out32.double(), ref) < 1.1 * norm_err(whole.double(), ref) + 1e-8 < K / 16 * 2.0**-23
+    out = gemm(a, b, **kw)
+    assert torch.equal(out, out32.to(torch.bfloat16))
+    acc = bf16(M, N)
+    want = (out32 + acc.float()).to(torch.bfloat16)
+    gemm(a, b, acc, accumulate=True, **kw)
+    assert torch.equal(acc, want)
+    wide = torch.zeros(M, N + 8, device=DEV, dtype=torch.bfloat16)
+    gemm(a, b, wide[:, :N], **kw)
+    assert torch.equal(wide[:, :N], out) and (wide[:, N:] == 0).all()
+    _lib.check_status("gemm")

@@ -29,7 +29,8 @@ namespace {
 // ------------------------------------------------------------------ the kernel library's entry points
 using P = const void*;
 struct Kernels {
-  int (*gemm)(P, P, P, int, int, int, int, int, int, int, int, int, int, P, P);
+  int (*gemm)(P, P, P, int, int, int, int, int, int, int, int, int, int, P, P, P);
+  int (*gemm_workspace)(int, int, int);
   int (*rmsnorm_parts)(int);
   int (*rmsnorm_fwd)(P, P, P, P, P, P, int, int, float, P);
   int (*rmsnorm_bwd)(P, P, P, P, P, P, P, P, int, int, int, P);
@@ -92,15 +93,23 @@ bool fits_int(int64_t v) { return v >= 0 && v <= INT32_MAX; }
 Tensor dense(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
 
 // ------------------------------------------------------------------ linear
+// out [M, N] = op(a) op(b): a is [M, K], or [K, M] with a_mn; b is [N, K], or [K, N] with b_mn.  All dense.
+void gemm(const Tensor& a, const Tensor& b, const Tensor& out, int64_t M, int64_t N, int64_t K, bool a_mn, bool b_mn) {
+  const int floats = kernels.gemm_workspace(M, N, K);
+  const Tensor workspace = floats ? at::empty({floats}, a.options().dtype(at::kFloat)) : Tensor();
+  check(kernels.gemm(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a_mn ? M : K, b_mn ? N : K, N, a_mn, b_mn, 0, 0,
+                     status_word(a), floats ? workspace.data_ptr() : nullptr, stream()),
+        "tft_gemm_bf16");
+  launched += floats ? 2 : 1;
+}
+
 struct Linear : public Function<Linear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w) {
     const int64_t N = w.size(0), K = w.size(1), M = x.numel() / K;
     auto sizes = x.sizes().vec();
     sizes.back() = N;
     Tensor y = at::empty(sizes, x.options());
-    check(kernels.gemm(x.data_ptr(), w.data_ptr(), y.data_ptr(), M, N, K, K, K, N, 0, 0, 0, 0, status_word(x), stream()),
-          "tft_gemm_bf16");
-    ++launched;
+    gemm(x, w, y, M, N, K, false, false);
     ctx->save_for_backward({x, w});
     return y;
   }
@@ -112,9 +121,7 @@ struct Linear : public Function<Linear> {
     Tensor dx, dw;
     if (ctx->needs_input_grad(0)) {
       dx = at::empty_like(x);
-      check(kernels.gemm(dy.data_ptr(), w.data_ptr(), dx.data_ptr(), M, K, N, N, K, K, 0, 1, 0, 0, status_word(x), stream()),
-            "tft_gemm_bf16");
-      ++launched;
+      gemm(dy, w, dx, M, K, N, false, true);
     }
     if (ctx->needs_input_grad(1)) {
       if (has_attr(w, "main_grad")) {  // given to the weight since the forward pass
@@ -123,9 +130,7 @@ struct Linear : public Function<Linear> {
         if (!g.is_none()) dw = g.cast<Tensor>();
       } else {
         dw = at::empty({N, K}, w.options());
-        check(kernels.gemm(dy.data_ptr(), x.data_ptr(), dw.data_ptr(), N, K, M, N, K, K, 1, 1, 0, 0, status_word(x), stream()),
-              "tft_gemm_bf16");
-        ++launched;
+        gemm(dy, x, dw, N, K, M, true, true);
       }
     }
     return {dx, dw};
@@ -330,6 +335,7 @@ void take(const py::dict& entries, const char* name, F& fn) {
 
 void setup(const py::dict& entries, py::object error, py::object status, py::object wgrad, py::object norm_target) {
   take(entries, "tft_gemm2_bf16", kernels.gemm);
+  take(entries, "tft_gemm2_workspace", kernels.gemm_workspace);
   take(entries, "tft_rmsnorm_bwd_parts", kernels.rmsnorm_parts);
   take(entries, "tft_rmsnorm_fwd", kernels.rmsnorm_fwd);
   take(entries, "tft_rmsnorm_bwd", kernels.rmsnorm_bwd);

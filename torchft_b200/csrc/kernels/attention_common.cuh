@@ -130,9 +130,7 @@ __device__ __forceinline__ void store_row_chunk(uint8_t* tile, int r, int c, con
 }
 
 // Stores 32 accumulator columns of each lane's row as bf16: `dst` is this lane's row at the first column, rows `stride`
-// elements apart, `rows_left` of them (counted from this lane's) exist.  Called by whole warps.  Four neighbouring lanes
-// first exchange their 16-byte pieces, so that one store instruction writes 64 contiguous bytes of eight rows instead of
-// 16 bytes of thirty-two.
+// elements apart, `rows_left` of them (counted from this lane's) exist.  Called by whole warps.
 __device__ __forceinline__ void store_rows32(const uint32_t (&a)[32], float mul, __nv_bfloat16* dst, long long stride,
                                              int rows_left) {
   const int lane = threadIdx.x & 31;
@@ -144,21 +142,7 @@ __device__ __forceinline__ void store_rows32(const uint32_t (&a)[32], float mul,
     u[t].z = pack_bf16(__uint_as_float(a[t * 8 + 4]) * mul, __uint_as_float(a[t * 8 + 5]) * mul);
     u[t].w = pack_bf16(__uint_as_float(a[t * 8 + 6]) * mul, __uint_as_float(a[t * 8 + 7]) * mul);
   }
-  // 4 x 4 transposition over the lanes: afterwards u[r] is piece (lane & 3) of row r of the four
-#pragma unroll
-  for (int step = 1; step <= 2; step <<= 1) {
-    const bool upper = lane & step;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int lo = step == 1 ? 2 * i : i, hi = lo + step;
-      uint4 give = upper ? u[lo] : u[hi];
-      give.x = __shfl_xor_sync(0xffffffffu, give.x, step);
-      give.y = __shfl_xor_sync(0xffffffffu, give.y, step);
-      give.z = __shfl_xor_sync(0xffffffffu, give.z, step);
-      give.w = __shfl_xor_sync(0xffffffffu, give.w, step);
-      if (upper) u[lo] = give; else u[hi] = give;
-    }
-  }
+  exchange_quad(u);
   const int piece = lane & 3;
 #pragma unroll
   for (int r = 0; r < 4; ++r)

@@ -259,6 +259,28 @@ __host__ __device__ constexpr uint32_t make_idesc_bf16(int m, int n, bool a_mn_m
          (static_cast<uint32_t>(m >> 4) << 24);
 }
 
+// Transposes the 4 x 4 pieces of 16 bytes that each group of four neighbouring lanes holds: before, u[i] is piece i of this
+// lane's row; afterwards u[r] is piece (lane & 3) of the row of the group's lane r.  Its own inverse; called by whole warps.
+// A store of rows that lie far apart then writes 64 contiguous bytes of eight rows per instruction instead of 16 bytes of
+// thirty-two.
+__device__ __forceinline__ void exchange_quad(uint4 (&u)[4]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int step = 1; step <= 2; step <<= 1) {
+    const bool upper = lane & step;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int lo = step == 1 ? 2 * i : i, hi = lo + step;
+      uint4 give = upper ? u[lo] : u[hi];
+      give.x = __shfl_xor_sync(0xffffffffu, give.x, step);
+      give.y = __shfl_xor_sync(0xffffffffu, give.y, step);
+      give.z = __shfl_xor_sync(0xffffffffu, give.z, step);
+      give.w = __shfl_xor_sync(0xffffffffu, give.w, step);
+      if (upper) u[lo] = give; else u[hi] = give;
+    }
+  }
+}
+
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);

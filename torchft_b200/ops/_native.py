@@ -20,7 +20,7 @@ from . import _lib
 _lock = threading.Lock()
 _module = None
 
-_ENTRIES = ("tft_gemm2_bf16", "tft_rmsnorm_bwd_parts", "tft_rmsnorm_fwd", "tft_rmsnorm_bwd", "tft_swiglu_fwd", "tft_swiglu_bwd",
+_ENTRIES = ("tft_gemm2_bf16", "tft_gemm2_workspace", "tft_rmsnorm_bwd_parts", "tft_rmsnorm_fwd", "tft_rmsnorm_bwd", "tft_swiglu_fwd", "tft_swiglu_bwd",
             "tft_xent", "tft_attn_fwd_pair", "tft_attn_bwd_tmem")
 
 

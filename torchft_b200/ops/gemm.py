@@ -54,12 +54,19 @@ def gemm(
     assert out.shape == (M, N) and out.stride(1) == 1
     if status is None:
         status = _lib.status_word(a.device)
-    fn = _lib.lib().tft_gemm2_bf16 if (impl or DEFAULT_IMPL) == "pair" else _lib.lib().tft_gemm_bf16
-    code = fn(
-        _lib.ptr(a), _lib.ptr(b), _lib.ptr(out), M, N, K, a.stride(0), b.stride(0), out.stride(0),
-        0 if a_kmajor else 1, 0 if b_kmajor else 1, 1 if out.dtype == torch.float32 else 0,
-        1 if accumulate else 0, _lib.ptr(status), _lib.stream_ptr(),
-    )
+    lib = _lib.lib()
+    args = (_lib.ptr(a), _lib.ptr(b), _lib.ptr(out), M, N, K, a.stride(0), b.stride(0), out.stride(0),
+            0 if a_kmajor else 1, 0 if b_kmajor else 1, 1 if out.dtype == torch.float32 else 0,
+            1 if accumulate else 0, _lib.ptr(status))
+    if (impl or DEFAULT_IMPL) == "pair":
+        # few tiles: the contraction is divided among the idle CTA pairs, whose partial sums need room
+        floats = lib.tft_gemm2_workspace(M, N, K)
+        workspace = torch.empty(floats, dtype=torch.float32, device=a.device) if floats else None
+        code = lib.tft_gemm2_bf16(*args, _lib.ptr(workspace), _lib.stream_ptr())
+        launches = 2 if floats else 1
+    else:
+        code = lib.tft_gemm_bf16(*args, _lib.stream_ptr())
+        launches = 1
     _lib.check(code, "tft_gemm_bf16")
-    _lib.count_launch()
+    _lib.count_launch(launches)
     return out
