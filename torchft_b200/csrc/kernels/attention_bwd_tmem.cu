@@ -325,43 +325,34 @@ int launch_dq_tmem(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorM
   return static_cast<int>(cudaGetLastError());
 }
 
-// ------------------------------------------------------------------ dK, dV (transposed scores)
+// ------------------------------------------------------------------ dK, dV (transposed scores), head dimension 128
 // An item is one query head of the group x one query tile.  Tensor-core order per item t:
 //
-//   dV(t) queries 0-63 | dV(t) 64-127 | S(t + LA) | dK(t) 0-63 | dK(t) 64-127 | dP(t + 1)
+//   dV(t) queries 0-63 | dV(t) 64-127 | S(t+1) | dK(t) 0-63 | dK(t) 64-127 | dP(t+1)
 //
 // The softmax threads work on the first 64 query columns of an item before the last 64 and announce the two halves
-// separately, so the gradient products start under the second half of the exponentials.  S(t + LA) follows dV(t)
-// directly and runs under the formation of dS(t); dP(t + 1) comes last, where nobody waits for it.  Head dimension 64
-// leaves room for two score regions (LA = 2): the scores of the next item are then ready before they are asked for.
-// With head dimension 128 the two accumulators take half of the tensor memory and LA is 1.
-// There the softmax threads set the pace, so two groups of eight warps take turns on the items; with head dimension 128
-// one group has the registers it needs and the score region is the limit.
-// What bounds it: the exponentials of an item take 1024 cycles of the MUFU unit (16 a cycle and SM) and the softmax threads
-// about half as long again for loads, dS, packing and stores; the four products take 2048 cycles at head dimension 128 and
-// 1024 at 64.  An item takes 2750 cycles (128: exponentials, then the last half of dV and the next S behind each other)
-// and 2300 (64: dS, dK and the next dP behind each other).  Measured, with the MMA warp as it is now and before it
-// stayed converged, and for attn_dkdv_split_kernel (P and dS through shared memory): 214, 233 and 275 us (one sequence
-// of 4096, 32/8 heads of 128); 92, 104 and 129 us (two of 2048, 32/8 heads of 64).
+// separately, so the gradient products start under the second half of the exponentials.  S(t+1) follows dV(t) directly and
+// runs under the formation of dS(t); dP(t+1) comes last, where nobody waits for it.  The two accumulators take half of the
+// tensor memory, which leaves one score region.
+// What bounds it: the exponentials of an item take 1024 cycles of the MUFU unit (16 a cycle and SM), the softmax threads
+// about half as long again for loads, dS, packing and stores, the four products 2048 cycles; an item takes 2750
+// (exponentials, then the last half of dV and the next S behind each other).  Measured, with the MMA warp as it is now and
+// before it stayed converged, and for attn_dkdv_split_kernel (P and dS through shared memory): 214, 233 and 275 us (one
+// sequence of 4096, 32/8 heads of 128).
 template <int HD>
 struct DkvTmemSmem {
-  static constexpr int LA = HD == 64 ? 2 : 1;  // score regions: how many items ahead S is issued
-  static constexpr int QST = LA + 1;           // Q(t) is read by dK(t) after S(t + LA) has been issued
-  static constexpr int DST = 2;
-  static constexpr int NG = LA;                // groups of 8 softmax warps that take turns
-  static constexpr int THREADS = 64 + NG * 256;
+  static constexpr int QST = 2, DST = 2;
+  static constexpr int THREADS = 64 + 256;
   static constexpr uint32_t TILE = BLK * HD * 2;
   static constexpr uint32_t K = 0, V = TILE, Q = 2 * TILE, DO = Q + QST * TILE;
-  static constexpr uint32_t STATS = DO + DST * TILE;  // float [groups][2 buffers][lse 128 | delta 128]
-  static constexpr uint32_t BARS = STATS + NG * 2 * 2 * BLK * 4;
+  static constexpr uint32_t STATS = DO + DST * TILE;  // float [2 buffers][lse 128 | delta 128]
+  static constexpr uint32_t BARS = STATS + 2 * 2 * BLK * 4;
   static constexpr uint32_t TOTAL = BARS + 256 + 1024;
 };
 enum DkvTmemBar {
-  TK_KV_FULL = 0, TK_Q_FULL0, TK_Q_EMPTY0 = TK_Q_FULL0 + 3, TK_DO_FULL0 = TK_Q_EMPTY0 + 3, TK_DO_EMPTY0 = TK_DO_FULL0 + 2,
-  TK_S_FULL0 = TK_DO_EMPTY0 + 2, TK_DP_FULL0 = TK_S_FULL0 + 2,
-  // one of each per group of softmax warps: P and dS of the first and of the last 64 query columns are stored
-  TK_P_LO0 = TK_DP_FULL0 + 2, TK_P_HI0 = TK_P_LO0 + 2, TK_DS_LO0 = TK_P_HI0 + 2, TK_DS_HI0 = TK_DS_LO0 + 2,
-  TK_ACC_DONE = TK_DS_HI0 + 2, NUM_TK_BARS
+  TK_KV_FULL = 0, TK_Q_FULL0 = 1, TK_Q_EMPTY0 = 3, TK_DO_FULL0 = 5, TK_DO_EMPTY0 = 7, TK_S_FULL = 9, TK_DP_FULL,
+  TK_P_LO, TK_P_HI, TK_DS_LO, TK_DS_HI,  // P and dS of the first and of the last 64 query columns are stored
+  TK_ACC_DONE, NUM_TK_BARS
 };
 
 // Column of k-step kk (16 of an item's 128 query columns) inside a 128-column region.  The thread of half h of a key row
@@ -392,7 +383,7 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
                       __nv_bfloat16* __restrict__ dV, int S, int Hq, int Hkv, long long lddk, long long lddv, float scale,
                       float scale_log2, int* status) {
   using L = DkvTmemSmem<HD>;
-  constexpr int LA = L::LA, QST = L::QST, DST = L::DST, NG = L::NG;
+  constexpr int QST = L::QST, DST = L::DST;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -411,7 +402,7 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
   const int n_items = G * (n_tiles - jt);  // (query head of the group, query tile at or after the key tile)
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < NUM_TK_BARS; ++i) mbar_init(bar(i), (i >= TK_P_LO0 && i < TK_ACC_DONE) ? 8 : 1);  // one arrival per warp of a group
+    for (int i = 0; i < NUM_TK_BARS; ++i) mbar_init(bar(i), (i >= TK_P_LO && i < TK_ACC_DONE) ? 8 : 1);  // one arrival per softmax warp
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tq);
@@ -428,8 +419,7 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
   // key rows on the lanes everywhere: S^T (later P^T) of item t, dP^T (later dS^T), the two accumulators
-  auto t_st = [&](int t) { return tmem_base + (LA == 2 ? static_cast<uint32_t>(t & 1) * 128u : 0u); };
-  const uint32_t t_dpt = tmem_base + LA * 128u, t_dv = t_dpt + 128u, t_dk = t_dv + HD;
+  const uint32_t t_st = tmem_base, t_dpt = tmem_base + 128u, t_dv = tmem_base + 256u, t_dk = t_dv + HD;
 
   if (warp == 0) {
     if (lane == 0) {
@@ -463,8 +453,8 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
         tc_fence_after();
         const uint32_t sq = base + L::Q + qs * L::TILE;
 #pragma unroll
-        for (int k = 0; k < HD / 16; ++k) umma_bf16_elect(leader, t_st(t), kmajor_desc(base + L::K, k), kmajor_desc(sq, k), idesc_s, k != 0);
-        umma_commit_elect(leader, bar(TK_S_FULL0 + t % LA));
+        for (int k = 0; k < HD / 16; ++k) umma_bf16_elect(leader, t_st, kmajor_desc(base + L::K, k), kmajor_desc(sq, k), idesc_s, k != 0);
+        umma_commit_elect(leader, bar(TK_S_FULL));
         return true;
       };
       auto issue_dp = [&](int t) -> bool {  // dP^T = V dO^T of item t
@@ -474,7 +464,7 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
         const uint32_t sdo = base + L::DO + ds * L::TILE;
 #pragma unroll
         for (int k = 0; k < HD / 16; ++k) umma_bf16_elect(leader, t_dpt, kmajor_desc(base + L::V, k), kmajor_desc(sdo, k), idesc_s, k != 0);
-        umma_commit_elect(leader, bar(TK_DP_FULL0 + t % NG));
+        umma_commit_elect(leader, bar(TK_DP_FULL));
         return true;
       };
       // acc (+)= A B over the item's query rows [64 half, 64 half + 64): A = P^T or dS^T from tensor memory
@@ -487,24 +477,22 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
       };
       bool ok = mbar_wait_warp(bar(TK_KV_FULL), 0, abort_flag);
       if (ok && n_items > 0) ok = issue_s(0) && issue_dp(0);
-      if (ok && LA == 2 && n_items > 1) ok = issue_s(1);
       for (int t = 0; t < n_items && ok; ++t) {
-        const int qs = t % QST, ds = t % DST, g = t % NG;
-        const uint32_t ph = (t / NG) & 1;
+        const int qs = t % QST, ds = t % DST;
         const uint32_t sq = base + L::Q + qs * L::TILE, sdo = base + L::DO + ds * L::TILE;
-        if (!mbar_wait_warp(bar(TK_P_LO0 + g), ph, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(TK_P_LO), t & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        issue_grad(t_dv, t_st(t), sdo, t, 0);
-        if (!mbar_wait_warp(bar(TK_P_HI0 + g), ph, abort_flag)) { ok = false; break; }
+        issue_grad(t_dv, t_st, sdo, t, 0);
+        if (!mbar_wait_warp(bar(TK_P_HI), t & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        issue_grad(t_dv, t_st(t), sdo, t, 1);
+        issue_grad(t_dv, t_st, sdo, t, 1);
         umma_commit_elect(leader, bar(TK_DO_EMPTY0 + ds));
         // in order behind dV(t), which was the last reader of the region
-        if (t + LA < n_items && !issue_s(t + LA)) { ok = false; break; }
-        if (!mbar_wait_warp(bar(TK_DS_LO0 + g), ph, abort_flag)) { ok = false; break; }
+        if (t + 1 < n_items && !issue_s(t + 1)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(TK_DS_LO), t & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         issue_grad(t_dk, t_dpt, sq, t, 0);
-        if (!mbar_wait_warp(bar(TK_DS_HI0 + g), ph, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(bar(TK_DS_HI), t & 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         issue_grad(t_dk, t_dpt, sq, t, 1);
         umma_commit_elect(leader, bar(TK_Q_EMPTY0 + qs));
@@ -514,11 +502,9 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
     }
   } else {
     const int q = warp & 3;
-    const int g = (warp - 2) >> 3;          // group: takes the items t with t % NG == g
-    const int gw = (warp - 2) & 7;          // warp inside the group
-    const int hf = gw >> 2;          // two threads per key row, each with 32 of the first and 32 of the last 64 query columns
+    const int hf = (warp - 2) >> 2;  // two threads per key row, each with 32 of the first and 32 of the last 64 query columns
     const int r = q * 32 + lane;     // key row inside the tile
-    const int e = gw * 32 + lane;    // 0..255: which statistic this thread fetches per item
+    const int e = (warp - 2) * 32 + lane;  // 0..255: which statistic this thread fetches per item
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     bool ok = true;
     // statistic of a query tile for this thread's slot: log-sum-exp (slots 0..127) or delta (128..255) of one
@@ -530,34 +516,28 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
       return qrow < S ? delta[at] : 0.f;
     };
     int it = jt, head = kv_head * G;
-    auto advance = [&]() {
+    float next_stat = fetch_stat(head, it);
+    for (int t = 0; t < n_items; ++t) {
+      const bool diag = it == jt;
+      const int q_end = S - it * BLK;                  // query columns at or beyond this one do not exist
+      const bool masked = diag || q_end < BLK;         // the same for the whole block
+      float* my_stats = stats + (t & 1) * 2 * BLK;
+      my_stats[e] = next_stat;
       if (++it == n_tiles) {
         it = jt;
         ++head;
       }
-    };
-    if (g == 1) advance();
-    float next_stat = g < n_items ? fetch_stat(head, it) : 0.f;
-    for (int t = g; t < n_items; t += NG) {
-      const uint32_t ph = (t / NG) & 1;
-      const bool diag = it == jt;
-      const int q_end = S - it * BLK;                  // query columns at or beyond this one do not exist
-      const bool masked = diag || q_end < BLK;         // the same for the whole block
-      float* my_stats = stats + (g * 2 + ph) * 2 * BLK;
-      my_stats[e] = next_stat;
-#pragma unroll
-      for (int i = 0; i < NG; ++i) advance();
-      if (t + NG < n_items) next_stat = fetch_stat(head, it);  // travels while this item is processed
-      ok = __all_sync(0xffffffffu, mbar_wait(bar(TK_S_FULL0 + t % LA), (t / LA) & 1, abort_flag)) && ok;
-      // every statistic of this item is in shared memory; all threads of the group leave together if one of them gave up
-      ok = !softmax_threads_any(g, !ok);
+      if (t + 1 < n_items) next_stat = fetch_stat(head, it);  // travels while this item is processed
+      ok = __all_sync(0xffffffffu, mbar_wait(bar(TK_S_FULL), t & 1, abort_flag)) && ok;
+      // every statistic of this item is in shared memory; all threads leave together if one of them gave up
+      ok = !softmax_threads_any(0, !ok);
       if (!ok) break;
       tc_fence_after();
       float p[2][32];
       {
         uint32_t sv[2][32];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) tmem_ld_32x32(t_st(t) + lane_addr + h * 64 + hf * 32, sv[h]);
+        for (int h = 0; h < 2; ++h) tmem_ld_32x32(t_st + lane_addr + h * 64 + hf * 32, sv[h]);
         tmem_ld_wait();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -576,50 +556,37 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
           }
           uint32_t packed[16];
           pack32(p[h], packed);
-          tmem_st_32x16(t_st(t) + lane_addr + c0, packed);  // over score columns this thread has already read
+          tmem_st_32x16(t_st + lane_addr + c0, packed);  // over score columns this thread has already read
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();  // the lanes' stores are ordered before the one arrival of the warp
-          if (lane == 0) mbar_arrive(bar((h == 0 ? TK_P_LO0 : TK_P_HI0) + g));
+          if (lane == 0) mbar_arrive(bar(h == 0 ? TK_P_LO : TK_P_HI));
         }
       }
-      ok = __all_sync(0xffffffffu, mbar_wait(bar(TK_DP_FULL0 + g), ph, abort_flag));  // acted upon at the next item's barrier
+      ok = __all_sync(0xffffffffu, mbar_wait(bar(TK_DP_FULL), t & 1, abort_flag));  // acted upon at the next item's barrier
       tc_fence_after();
       {
-        // one group: all of dP in flight at once.  Two groups have 96 registers a thread, so 16 columns at a time; the other
-        // group's work hides the waits.
-        constexpr int STEP = NG == 1 ? 64 : 16;
-        uint32_t dv[STEP];
-        if constexpr (NG == 1) {
-          tmem_ld_32x32(t_dpt + lane_addr + hf * 32, *reinterpret_cast<uint32_t(*)[32]>(&dv[0]));
-          tmem_ld_32x32(t_dpt + lane_addr + 64 + hf * 32, *reinterpret_cast<uint32_t(*)[32]>(&dv[32]));
-          tmem_ld_wait();
-        }
+        uint32_t dv[2][32];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) tmem_ld_32x32(t_dpt + lane_addr + h * 64 + hf * 32, dv[h]);
+        tmem_ld_wait();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int c0 = h * 64 + hf * 32;
-          uint32_t packed[16];
 #pragma unroll
           for (int i4 = 0; i4 < 8; ++i4) {
-            if constexpr (NG == 2) {
-              if (i4 % 4 == 0) {
-                tmem_ld_32x16(t_dpt + lane_addr + c0 + i4 * 4, *reinterpret_cast<uint32_t(*)[16]>(&dv[0]));
-                tmem_ld_wait();
-              }
-            }
             const float4 dl = *reinterpret_cast<const float4*>(my_stats + BLK + c0 + i4 * 4);
             const float dlv[4] = {dl.x, dl.y, dl.z, dl.w};
-            float ds[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) ds[u] = p[h][i4 * 4 + u] * (__uint_as_float(dv[(h * 32 + i4 * 4 + u) % STEP]) - dlv[u]);
-            packed[i4 * 2] = pack_bf16(ds[0], ds[1]);
-            packed[i4 * 2 + 1] = pack_bf16(ds[2], ds[3]);
+            for (int u = 0; u < 4; ++u) p[h][i4 * 4 + u] *= __uint_as_float(dv[h][i4 * 4 + u]) - dlv[u];
           }
+          uint32_t packed[16];
+          pack32(p[h], packed);
           tmem_st_32x16(t_dpt + lane_addr + c0, packed);
           tmem_st_wait();
           tc_fence_before();
           __syncwarp();
-          if (lane == 0) mbar_arrive(bar((h == 0 ? TK_DS_LO0 : TK_DS_HI0) + g));
+          if (lane == 0) mbar_arrive(bar(h == 0 ? TK_DS_LO : TK_DS_HI));
         }
       }
     }
@@ -629,11 +596,263 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
         tc_fence_after();
         const int krow = jt * BLK + r;
         const long long tok = static_cast<long long>(batch) * S + krow;
-        if (NG == 1 || g == 0)
-          store_acc<HD / 2>(t_dv + lane_addr + hf * (HD / 2), dV + tok * lddv + kv_head * HD + hf * (HD / 2), lddv, 1.f, S - krow);
-        if (NG == 1 || g == 1)
-          store_acc<HD / 2>(t_dk + lane_addr + hf * (HD / 2), dK + tok * lddk + kv_head * HD + hf * (HD / 2), lddk, scale, S - krow);
+        store_acc<HD / 2>(t_dv + lane_addr + hf * (HD / 2), dV + tok * lddv + kv_head * HD + hf * (HD / 2), lddv, 1.f, S - krow);
+        store_acc<HD / 2>(t_dk + lane_addr + hf * (HD / 2), dK + tok * lddk + kv_head * HD + hf * (HD / 2), lddk, scale, S - krow);
       }
+    }
+    tc_fence_before();
+  }
+
+  __syncthreads();
+  if (*abort_flag) {
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000LL) { }
+    if (threadIdx.x == 0 && status) atomicCAS(status, 0, static_cast<int>(kTimeoutBarrier));
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// ------------------------------------------------------------------ dK, dV at head dimension 64: two half pipelines
+// Products are cheap here (1152 cycles an item) and the softmax threads set the pace, so two groups of eight warps take the
+// two halves of every item's query columns, each with its own hand-over of P, dP and dS.  dP^T is computed per half
+// (N = 64), so a half's region is free as soon as its own dK product has been issued, and the groups drift half an item
+// apart: one forms dS (FMA, packing) under the exponentials (MUFU) of the other.  Tensor-core order per item t:
+//
+//   dV(t) half 0 | dK(t-1) half 1 | dP(t) half 1 | dV(t) half 1 | S(t+2) | dK(t) half 0 | dP(t+1) half 0
+//
+// Two sequences of 2048, 32/8 heads of 64: 83 us; 90 with the groups taking turns on whole items (one dP region makes dS, dK
+// and the next dP a chain), 101 with sixteen warps on one item, 104 with eight, 129 for attn_dkdv_split_kernel.
+struct DkvHalves {
+  static constexpr int HD = 64, QST = 4, DST = 3;
+  static constexpr int THREADS = 64 + 512;
+  static constexpr uint32_t TILE = BLK * HD * 2;
+  static constexpr uint32_t K = 0, V = TILE, Q = 2 * TILE, DO = Q + QST * TILE;
+  static constexpr uint32_t STATS = DO + DST * TILE;  // float [groups][2 buffers][lse 64 | delta 64]
+  static constexpr uint32_t BARS = STATS + 2 * 2 * BLK * 4;
+  static constexpr uint32_t TOTAL = BARS + 256 + 1024;
+};
+enum DkvHalvesBar {
+  TH_KV_FULL = 0, TH_Q_FULL0 = 1, TH_Q_EMPTY0 = 5, TH_DO_FULL0 = 9, TH_DO_EMPTY0 = 12, TH_S_FULL0 = 15, TH_DP_FULL0 = 17,
+  TH_P0 = 19, TH_DS0 = 21, TH_ACC_DONE = 23, NUM_TH_BARS = 24
+};
+
+__global__ void __launch_bounds__(DkvHalves::THREADS, 1)
+attn_dkdv_halves_kernel(const __grid_constant__ CUtensorMap tq, const __grid_constant__ CUtensorMap tk,
+                      const __grid_constant__ CUtensorMap tv, const __grid_constant__ CUtensorMap tdo,
+                      const float* __restrict__ LSE, const float* __restrict__ delta, __nv_bfloat16* __restrict__ dK,
+                      __nv_bfloat16* __restrict__ dV, int S, int Hq, int Hkv, long long lddk, long long lddv, float scale,
+                      float scale_log2, int* status) {
+  using L = DkvHalves;
+  constexpr int HD = L::HD, QST = L::QST, DST = L::DST;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  uint8_t* smem = smem_raw + (base - raw);
+  const uint32_t bar0 = base + L::BARS;
+  auto bar = [&](int i) { return bar0 + 8u * i; };
+  volatile uint32_t* tmem_holder = reinterpret_cast<volatile uint32_t*>(smem + L::BARS + 8 * NUM_TH_BARS);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::BARS + 8 * NUM_TH_BARS + 8);
+  float* stats = reinterpret_cast<float*>(smem + L::STATS);
+
+  const int warp = uniform_warp_index(), lane = threadIdx.x & 31;
+  const int n_tiles = (S + BLK - 1) / BLK;
+  const int jt = blockIdx.x / Hkv;  // key tile; early key tiles have the most work and come first
+  const int kv_head = blockIdx.x % Hkv, batch = blockIdx.y;
+  const int G = Hq / Hkv;
+  const int n_items = G * (n_tiles - jt);  // (query head of the group, query tile at or after the key tile)
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < NUM_TH_BARS; ++i) mbar_init(bar(i), (i >= TH_P0 && i < TH_ACC_DONE) ? 8 : 1);  // one arrival per warp of a group
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tq);
+    tma_prefetch_desc(&tk);
+    tma_prefetch_desc(&tv);
+    tma_prefetch_desc(&tdo);
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(const_cast<uint32_t*>(tmem_holder)), 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_holder;
+  // key rows on the lanes everywhere: S^T (later P^T) of item t, dP^T (later dS^T), the two accumulators
+  auto t_st = [&](int t) { return tmem_base + static_cast<uint32_t>(t & 1) * 128u; };
+  const uint32_t t_dpt = tmem_base + 256u, t_dv = t_dpt + 128u, t_dk = t_dv + HD;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      mbar_expect_tx(bar(TH_KV_FULL), 2 * L::TILE);
+      load_tile<HD>(base + L::K, &tk, bar(TH_KV_FULL), kv_head, jt * BLK, batch);
+      load_tile<HD>(base + L::V, &tv, bar(TH_KV_FULL), kv_head, jt * BLK, batch);
+      int it = jt, head = kv_head * G;
+      for (int t = 0; t < n_items; ++t) {
+        const int qs = t % QST, ds = t % DST;
+        if (!mbar_wait(bar(TH_Q_EMPTY0 + qs), ((t / QST) & 1) ^ 1, abort_flag)) break;
+        mbar_expect_tx(bar(TH_Q_FULL0 + qs), L::TILE);
+        load_tile<HD>(base + L::Q + qs * L::TILE, &tq, bar(TH_Q_FULL0 + qs), head, it * BLK, batch);
+        if (!mbar_wait(bar(TH_DO_EMPTY0 + ds), ((t / DST) & 1) ^ 1, abort_flag)) break;
+        mbar_expect_tx(bar(TH_DO_FULL0 + ds), L::TILE);
+        load_tile<HD>(base + L::DO + ds * L::TILE, &tdo, bar(TH_DO_FULL0 + ds), head, it * BLK, batch);
+        if (++it == n_tiles) {
+          it = jt;
+          ++head;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    const uint32_t leader = elect_one();
+    constexpr uint32_t idesc_s = make_idesc_bf16(BLK, BLK, false, false);  // 128 keys x 128 queries
+    constexpr uint32_t idesc_dp = make_idesc_bf16(BLK, 64, false, false);  // 128 keys x 64 queries
+    constexpr uint32_t idesc_g = make_idesc_bf16(BLK, HD, false, true);
+    auto issue_s = [&](int t) -> bool {  // S^T = K Q^T of item t
+      const int qs = t % QST;
+      if (!mbar_wait_warp(bar(TH_Q_FULL0 + qs), (t / QST) & 1, abort_flag)) return false;
+      tc_fence_after();
+      const uint32_t sq = base + L::Q + qs * L::TILE;
+#pragma unroll
+      for (int k = 0; k < HD / 16; ++k) umma_bf16_elect(leader, t_st(t), kmajor_desc(base + L::K, k), kmajor_desc(sq, k), idesc_s, k != 0);
+      umma_commit_elect(leader, bar(TH_S_FULL0 + (t & 1)));
+      return true;
+    };
+    auto issue_dp = [&](int t, int half) -> bool {  // dP^T = V dO^T for the item's query rows [64 half, 64 half + 64)
+      const int ds = t % DST;
+      if (!mbar_wait_warp(bar(TH_DO_FULL0 + ds), (t / DST) & 1, abort_flag)) return false;
+      tc_fence_after();
+      const uint32_t sdo = base + L::DO + ds * L::TILE + half * 8192;
+#pragma unroll
+      for (int k = 0; k < HD / 16; ++k)
+        umma_bf16_elect(leader, t_dpt + half * 64, kmajor_desc(base + L::V, k), kmajor_desc(sdo, k), idesc_dp, k != 0);
+      umma_commit_elect(leader, bar(TH_DP_FULL0 + half));
+      return true;
+    };
+    // acc (+)= A B over one half's query rows, once its group has stored A (P^T or dS^T) in tensor memory
+    auto issue_grad = [&](int ready, int t, int half, uint32_t acc, uint32_t a_region, uint32_t b_tile) -> bool {
+      if (!mbar_wait_warp(bar(ready + half), t & 1, abort_flag)) return false;
+      tc_fence_after();
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        const int k = half * 4 + kk;
+        umma_bf16_ts_elect(leader, acc, dkv_kstep(a_region, k), mnmajor_desc(b_tile, k), idesc_g, (t | k) != 0);
+      }
+      return true;
+    };
+    auto q_tile = [&](int t) { return base + L::Q + (t % QST) * L::TILE; };
+    auto do_tile = [&](int t) { return base + L::DO + (t % DST) * L::TILE; };
+    auto last_of_item = [&](int t) -> bool {  // dK of the second half: the last reader of the item's Q
+      if (!issue_grad(TH_DS0, t, 1, t_dk, t_dpt, q_tile(t))) return false;
+      umma_commit_elect(leader, bar(TH_Q_EMPTY0 + t % QST));
+      return true;
+    };
+    bool ok = mbar_wait_warp(bar(TH_KV_FULL), 0, abort_flag) && issue_s(0) && issue_dp(0, 0);
+    if (ok && n_items > 1) ok = issue_s(1);
+    for (int t = 0; t < n_items && ok; ++t) {
+      ok = issue_grad(TH_P0, t, 0, t_dv, t_st(t), do_tile(t)) && (t == 0 || last_of_item(t - 1)) && issue_dp(t, 1) &&
+           issue_grad(TH_P0, t, 1, t_dv, t_st(t), do_tile(t));
+      if (!ok) break;
+      umma_commit_elect(leader, bar(TH_DO_EMPTY0 + t % DST));
+      // in order behind dV(t), which was the last reader of the region
+      if (t + 2 < n_items && !issue_s(t + 2)) { ok = false; break; }
+      ok = issue_grad(TH_DS0, t, 0, t_dk, t_dpt, q_tile(t)) && (t + 1 == n_items || issue_dp(t + 1, 0));
+    }
+    if (ok && last_of_item(n_items - 1)) umma_commit_elect(leader, bar(TH_ACC_DONE));
+  } else {
+    const int q = warp & 3;
+    const int g = (warp - 2) >> 3;         // group: query columns [64 g, 64 g + 64) of every item
+    const int gw = (warp - 2) & 7;         // warp inside the group
+    const int hf = gw >> 2;                // two threads per key row, 32 columns each
+    const int r = q * 32 + lane;           // key row inside the tile
+    const int e = gw * 32 + lane;          // the first 128 fetch the statistics of the group's 64 query rows
+    const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
+    const int c0 = g * 64 + hf * 32;       // first column of this thread
+    bool ok = true;
+    // log-sum-exp (slots 0..63) or delta (64..127) of one query row; +inf as log-sum-exp of a row beyond the sequence turns
+    // its probabilities into zeros
+    auto fetch_stat = [&](int head, int it) -> float {
+      const int qrow = it * BLK + g * 64 + (e & 63);
+      const long long at = (static_cast<long long>(batch) * Hq + head) * S + qrow;
+      if (e < 64) return qrow < S ? LSE[at] : INFINITY;
+      return qrow < S ? delta[at] : 0.f;
+    };
+    int it = jt, head = kv_head * G;
+    float next_stat = e < 128 ? fetch_stat(head, it) : 0.f;
+    for (int t = 0; t < n_items; ++t) {
+      const bool diag = it == jt;
+      const int q_end = S - it * BLK;                  // query columns at or beyond this one do not exist
+      const bool masked = diag || q_end < BLK;         // the same for the whole block
+      float* my_stats = stats + (g * 2 + (t & 1)) * BLK;
+      if (e < 128) my_stats[e] = next_stat;
+      if (++it == n_tiles) {
+        it = jt;
+        ++head;
+      }
+      if (t + 1 < n_items && e < 128) next_stat = fetch_stat(head, it);  // travels while this item is processed
+      ok = mbar_wait_warp(bar(TH_S_FULL0 + (t & 1)), (t >> 1) & 1, abort_flag) && ok;
+      // every statistic of this item is in shared memory; all threads of the group leave together if one of them gave up
+      ok = !softmax_threads_any(g, !ok);
+      if (!ok) break;
+      tc_fence_after();
+      float p[32];
+      {
+        uint32_t sv[32];
+        tmem_ld_32x32(t_st(t) + lane_addr + c0, sv);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i4 = 0; i4 < 8; ++i4) {
+          const float4 ls = *reinterpret_cast<const float4*>(my_stats + hf * 32 + i4 * 4);
+          const float lsv[4] = {ls.x, ls.y, ls.z, ls.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) p[i4 * 4 + u] = fast_exp2(__uint_as_float(sv[i4 * 4 + u]) * scale_log2 - lsv[u]);
+        }
+        if (masked) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)  // causal: query column >= key row
+            if ((diag && c0 + i < r) || c0 + i >= q_end) p[i] = 0.f;
+        }
+        uint32_t packed[16];
+        pack32(p, packed);
+        tmem_st_32x16(t_st(t) + lane_addr + c0, packed);  // over score columns this thread has already read
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();  // the lanes' stores are ordered before the one arrival of the warp
+        if (lane == 0) mbar_arrive(bar(TH_P0 + g));
+      }
+      ok = mbar_wait_warp(bar(TH_DP_FULL0 + g), t & 1, abort_flag);  // acted upon at the next item's barrier
+      tc_fence_after();
+      {
+        uint32_t dv[32];
+        tmem_ld_32x32(t_dpt + lane_addr + c0, dv);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i4 = 0; i4 < 8; ++i4) {
+          const float4 dl = *reinterpret_cast<const float4*>(my_stats + 64 + hf * 32 + i4 * 4);
+          const float dlv[4] = {dl.x, dl.y, dl.z, dl.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) p[i4 * 4 + u] *= __uint_as_float(dv[i4 * 4 + u]) - dlv[u];
+        }
+        uint32_t packed[16];
+        pack32(p, packed);
+        tmem_st_32x16(t_dpt + lane_addr + c0, packed);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(TH_DS0 + g));
+      }
+    }
+    if (ok && mbar_wait_warp(bar(TH_ACC_DONE), 0, abort_flag)) {
+      tc_fence_after();
+      const int krow = jt * BLK + r, col = hf * (HD / 2);
+      const long long tok = static_cast<long long>(batch) * S + krow;
+      if (g == 0)
+        store_acc<HD / 2>(t_dv + lane_addr + col, dV + tok * lddv + kv_head * HD + col, lddv, 1.f, S - krow);
+      else
+        store_acc<HD / 2>(t_dk + lane_addr + col, dK + tok * lddk + kv_head * HD + col, lddk, scale, S - krow);
     }
     tc_fence_before();
   }
@@ -655,17 +874,29 @@ template <int HD>
 int launch_dkdv_tmem(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
                      const float* lse, const float* delta, void* dk, void* dv, int B, int S, int Hq, int Hkv,
                      long long lddk, long long lddv, float scale, int* status, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_dkdv_tmem_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         DkvTmemSmem<HD>::TOTAL);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
   const int n_tiles = (S + BLK - 1) / BLK;
-  attn_dkdv_tmem_kernel<HD><<<dim3(n_tiles * Hkv, B, 1), DkvTmemSmem<HD>::THREADS, DkvTmemSmem<HD>::TOTAL, stream>>>(
-      tq, tk, tv, tdo, lse, delta, static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), S, Hq, Hkv, lddk,
-      lddv, scale, scale * 1.4426950408889634f, status);
+  const dim3 grid(n_tiles * Hkv, B, 1);
+  static bool configured = false;
+  if constexpr (HD == 64) {
+    if (!configured) {
+      const cudaError_t e = cudaFuncSetAttribute(attn_dkdv_halves_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DkvHalves::TOTAL);
+      if (e != cudaSuccess) return static_cast<int>(e);
+      configured = true;
+    }
+    attn_dkdv_halves_kernel<<<grid, DkvHalves::THREADS, DkvHalves::TOTAL, stream>>>(
+        tq, tk, tv, tdo, lse, delta, static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), S, Hq, Hkv, lddk,
+        lddv, scale, scale * 1.4426950408889634f, status);
+  } else {
+    if (!configured) {
+      const cudaError_t e = cudaFuncSetAttribute(attn_dkdv_tmem_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 DkvTmemSmem<HD>::TOTAL);
+      if (e != cudaSuccess) return static_cast<int>(e);
+      configured = true;
+    }
+    attn_dkdv_tmem_kernel<HD><<<grid, DkvTmemSmem<HD>::THREADS, DkvTmemSmem<HD>::TOTAL, stream>>>(
+        tq, tk, tv, tdo, lse, delta, static_cast<__nv_bfloat16*>(dk), static_cast<__nv_bfloat16*>(dv), S, Hq, Hkv, lddk,
+        lddv, scale, scale * 1.4426950408889634f, status);
+  }
   return static_cast<int>(cudaGetLastError());
 }
 
