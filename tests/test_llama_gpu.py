@@ -100,6 +100,34 @@ def test_engine_trains_and_state_round_trips():
     torch.testing.assert_close(engine.flat_param.float(), engine2.flat_param.float(), rtol=2e-2, atol=2e-3)
 
 
+def test_engine_gradients_with_checkpointed_blocks():
+    """Activation checkpointing runs the same kernels on the same values again: every gradient is in its buffer, equal bit for
+    bit to the run without it (the embedding's apart, whose sum is taken with atomics)."""
+    from torch.utils.checkpoint import checkpoint
+
+    from torchft_b200.models.llama import Llama, LlamaConfig
+    from torchft_b200.parallel.hsdp import HSDPEngine
+
+    cfg = LlamaConfig.tiny()
+    torch.manual_seed(0)
+    tokens = torch.randint(cfg.vocab_size, (2, 256), device="cuda")
+    targets = torch.randint(cfg.vocab_size, (2, 256), device="cuda")
+    grads = []
+    for checkpointed in (False, True):
+        model = Llama(cfg, device="cuda")
+        model.init_weights(seed=0)
+        engine = HSDPEngine(model, model.units(), lr=1e-3)
+        if checkpointed:
+            for layer in model.layers:
+                layer.forward = lambda *a, forward=layer.forward: checkpoint(forward, *a, use_reentrant=False)
+        engine.train_step(tokens, targets)
+        torch.cuda.synchronize()
+        assert all(p.grad is None for p in model.parameters())
+        grads.append({n: p.main_grad.clone() for n, p in model.named_parameters() if n != "tok_embeddings"})
+    for name, grad in grads[0].items():
+        assert grad.any() and torch.equal(grad, grads[1][name]), name
+
+
 def test_forward_backward_is_cuda_graph_capturable():
     """The kernels make no call that is illegal during stream capture: a whole forward + backward
     of the model replays from a CUDA graph with the gradients of the eager run."""

@@ -60,11 +60,14 @@ def test_calls_that_stay_with_the_python_nodes():
     assert m.linear(x, w) is not None
     wide = torch.zeros(16, 128, device=DEV, dtype=torch.bfloat16)
     odd = torch.zeros(16 * 64 + 1, device=DEV, dtype=torch.bfloat16)[1:].view(16, 64)
-    marked = leaf(32, 64)
-    marked.main_grad = torch.zeros_like(marked)
+    marked, marked_norm = leaf(32, 64), leaf(256)
+    for weight in (marked, marked_norm):
+        weight.main_grad = torch.zeros_like(weight)
     for a, b in ((wide[:, :64], w), (odd, w), (x.float(), w), (x.cpu(), w), (x, marked), (leaf(16, 60), leaf(32, 60)), (x[:0], w)):
         assert m.linear(a, b) is None
     assert m.rmsnorm(leaf(4, 264), leaf(264), 1e-5) is None  # a width that the kernel has no split for
+    rows = leaf(4, 256)
+    assert m.rmsnorm(rows, marked_norm, 1e-5) is None and m.add_rmsnorm(rows, rows, marked_norm, 1e-5) is None
     assert m.swiglu(leaf(4, 24)) is None
     torch.manual_seed(0)
     strided = torch.randn(16, 128, device=DEV).to(torch.bfloat16)[:, ::2]
@@ -113,6 +116,32 @@ def test_saved_tensor_hooks_and_late_gradient_buffers():
     assert torch.isfinite(w.main_grad).all() and w.main_grad_initialized
     want = dy.float().t() @ F.rmsnorm(x, n.detach().clone()).detach().float()
     assert (w.main_grad.float() - want).norm() < 8e-3 * want.norm()  # one rounding of the sum to bf16
+
+
+@pytest.mark.parametrize("late", [False, True])
+@pytest.mark.parametrize("name", ["linear", "rmsnorm", "add_rmsnorm"])
+def test_gradient_buffers_under_saved_tensor_hooks(name, late):
+    """What the hooks unpack is a copy without the weight's attributes: the gradient goes to the weight's buffer all the same,
+    given to it before the forward pass or after it."""
+    from torchft_b200.ops import attention as A
+    from torchft_b200.ops import functional as F
+
+    torch.manual_seed(0)
+    fn, _, inputs = CASES[name](F, A)
+    w = inputs[-1]
+    out = fn(*inputs)
+    out = out[0] if isinstance(out, tuple) else out
+    dy = torch.randn_like(out)
+    (want,) = torch.autograd.grad(out, (w,), dy)
+    buffer = torch.full_like(w, float("nan"))
+    if not late:
+        w.main_grad = buffer
+    with torch.autograd.graph.save_on_cpu():
+        out = fn(*inputs)
+    w.main_grad = buffer
+    (out[0] if isinstance(out, tuple) else out).backward(dy)
+    assert w.grad is None and w.main_grad_initialized
+    assert torch.equal(buffer, want)
 
 
 def test_cross_entropy_matches_the_python_node():

@@ -83,10 +83,15 @@ bool plain(const py::handle& h, at::ScalarType type = at::kBFloat16) {
   return t.is_cuda() && t.scalar_type() == type && t.has_storage() && t.layout() == at::kStrided && !t.is_neg() && !t.is_conj() &&
          t.get_device() < kMaxDevices && t.numel() > 0 && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 && !t._fw_grad(0).defined();
 }
-bool has_attr(const Tensor& t, const char* name) {
+// A weight that carries `main_grad` at the forward pass belongs to the Python nodes.  The buffer may also be given to it
+// between the passes, and the weight's own attributes decide: what a saved-tensor hook (offloading, activation
+// checkpointing) unpacks is another tensor without them.  So the weight itself travels beside the saved tensors.
+bool has_main_grad(py::handle weight) { return PyObject_HasAttrString(weight.ptr(), "main_grad") != 0; }
+void keep_weight(AutogradContext* ctx, const Tensor& w) { ctx->saved_data["weight"] = w; }
+Tensor kept_weight(AutogradContext* ctx) { return ctx->saved_data["weight"].toTensor(); }
+bool has_main_grad(const Tensor& weight) {
   py::gil_scoped_acquire gil;
-  const py::object o = py::reinterpret_steal<py::object>(THPVariable_Wrap(t));
-  return PyObject_HasAttrString(o.ptr(), name) != 0;
+  return has_main_grad(py::reinterpret_steal<py::object>(THPVariable_Wrap(weight)));
 }
 bool fits_int(int64_t v) { return v >= 0 && v <= INT32_MAX; }
 
@@ -111,6 +116,7 @@ struct Linear : public Function<Linear> {
     Tensor y = at::empty(sizes, x.options());
     gemm(x, w, y, M, N, K, false, false);
     ctx->save_for_backward({x, w});
+    keep_weight(ctx, w);
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -124,9 +130,10 @@ struct Linear : public Function<Linear> {
       gemm(dy, w, dx, M, K, N, false, true);
     }
     if (ctx->needs_input_grad(1)) {
-      if (has_attr(w, "main_grad")) {  // given to the weight since the forward pass
+      const Tensor weight = kept_weight(ctx);
+      if (has_main_grad(weight)) {  // given to it since the forward pass
         py::gil_scoped_acquire gil;
-        const py::object g = py::handle(linear_wgrad)(w, dy.view({M, N}), x.view({M, K}));
+        const py::object g = py::handle(linear_wgrad)(weight, dy.view({M, N}), x.view({M, K}));
         if (!g.is_none()) dw = g.cast<Tensor>();
       } else {
         dw = at::empty({N, K}, w.options());
@@ -144,7 +151,7 @@ py::object linear(py::handle hx, py::handle hw) {
       w.size(1) % 8 || !fits_int(x.numel() / w.size(1)) || !fits_int(w.size(0)) || !fits_int(w.size(1)) ||
       x.get_device() != w.get_device())
     return py::none();
-  if (PyObject_HasAttrString(hw.ptr(), "main_grad") || PyObject_HasAttrString(hw.ptr(), "gather_comm")) return py::none();
+  if (has_main_grad(hw) || PyObject_HasAttrString(hw.ptr(), "gather_comm")) return py::none();
   return py::cast(Linear::apply(x, w));
 }
 
@@ -157,15 +164,15 @@ bool norm_dim(int64_t dim) {
 }
 
 // (dx, dw) of y = rmsnorm(h) * w; dres is added to dx.
-std::pair<Tensor, Tensor> norm_backward(const Tensor& grad_y, const Tensor& h, const Tensor& w, const Tensor& rstd,
-                                        const Tensor& grad_h) {
+std::pair<Tensor, Tensor> norm_backward(const Tensor& weight, const Tensor& grad_y, const Tensor& h, const Tensor& w,
+                                        const Tensor& rstd, const Tensor& grad_h) {
   const int64_t dim = h.size(-1), rows = h.numel() / dim;
   const Tensor dy = dense(grad_y), dres = grad_h.defined() ? dense(grad_h) : grad_h;
   Tensor dx = at::empty_like(h), dw, out;
   bool accumulate = false;
-  if (has_attr(w, "main_grad")) {
+  if (has_main_grad(weight)) {  // given to it since the forward pass
     py::gil_scoped_acquire gil;
-    const py::tuple target = py::handle(norm_wgrad_target)(w);
+    const py::tuple target = py::handle(norm_wgrad_target)(weight);
     if (!target[0].is_none()) out = target[0].cast<Tensor>();
     accumulate = target[1].cast<bool>();
   }
@@ -186,11 +193,12 @@ struct RMSNorm : public Function<RMSNorm> {
           "tft_rmsnorm_fwd");
     ++launched;
     ctx->save_for_backward({x, w, rstd});
+    keep_weight(ctx, w);
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
-    auto [dx, dw] = norm_backward(grads[0], s[0], s[1], s[2], Tensor());
+    auto [dx, dw] = norm_backward(kept_weight(ctx), grads[0], s[0], s[1], s[2], Tensor());
     return {dx, dw, Tensor()};
   }
 };
@@ -204,6 +212,7 @@ struct AddRMSNorm : public Function<AddRMSNorm> {
           "tft_rmsnorm_fwd");
     ++launched;
     ctx->save_for_backward({h, w, rstd});
+    keep_weight(ctx, w);
     return {y, h};
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -211,7 +220,7 @@ struct AddRMSNorm : public Function<AddRMSNorm> {
     // an output that took no part in the loss arrives as zeros, as in the Python node
     const Tensor dy = grads[0].defined() ? grads[0] : at::zeros_like(s[0]);
     const Tensor dh = grads[1].defined() ? grads[1] : at::zeros_like(s[0]);
-    auto [dx, dw] = norm_backward(dy, s[0], s[1], s[2], dh);
+    auto [dx, dw] = norm_backward(kept_weight(ctx), dy, s[0], s[1], s[2], dh);
     return {dx, dx, dw, Tensor()};
   }
 };
@@ -220,7 +229,7 @@ bool plain_norm(py::handle hx, py::handle hw) {
   if (!plain(hx) || !plain(hw) || !plain_context()) return false;
   const Tensor &x = THPVariable_Unpack(hx.ptr()), &w = THPVariable_Unpack(hw.ptr());
   return x.dim() >= 1 && w.dim() == 1 && x.size(-1) == w.size(0) && x.is_contiguous() && w.is_contiguous() && norm_dim(w.size(0)) &&
-         fits_int(x.numel() / w.size(0)) && x.get_device() == w.get_device();
+         fits_int(x.numel() / w.size(0)) && x.get_device() == w.get_device() && !has_main_grad(hw);
 }
 py::object rmsnorm(py::handle hx, py::handle hw, double eps) {
   if (!plain_norm(hx, hw)) return py::none();
