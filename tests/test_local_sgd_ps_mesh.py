@@ -268,3 +268,20 @@ def test_fsdp2_over_managed_mesh_two_processes():
     port = probe.port
     del probe
     mp.spawn(_fsdp_worker, args=(2, port), nprocs=2, join=True)
+
+
+@pytest.mark.parametrize("shape", [(6, 8), (8, 6), (48,), (7, 8), (5, 8)])
+def test_outer_step_table_covers_the_buckets_and_no_more(shape):
+    """Sizes come from the buckets whatever has become of a parameter; one of another shape is reached through its view."""
+    from torchft_b200.local_sgd import _FlatBuckets
+    from torchft_b200.ops.outer_step import FusedOuterStep
+
+    params = [torch.nn.Parameter(torch.randn(s)) for s in ((6, 8), (16,))]
+    backup, comm = _FlatBuckets(params, None, False), _FlatBuckets(params, None, False)
+    fused = FusedOuterStep(params, backup, comm, torch.optim.SGD(params, lr=0.7, momentum=0.9))
+    params[0].data = torch.randn(shape)
+    ptrs, offs, sizes, n, packed = fused._table(next(iter(comm.flat)))
+    assert list(sizes) == [48, 16] and list(offs) == [0, 48] and n == 2
+    same = shape == (6, 8)
+    assert packed == ([] if same else [0])
+    assert ptrs[0] == (params[0] if same else comm.views[0]).data_ptr() and ptrs[1] == params[1].data_ptr()

@@ -364,6 +364,32 @@ def test_outer_step_reads_and_writes_the_parameters_in_place(dtype, momentum, ne
             old[i] = p.detach().clone()
 
 
+@pytest.mark.parametrize("shape", [(8, 6), (48,), (7, 8), (5, 8)])
+def test_outer_step_refuses_a_parameter_of_another_shape(shape):
+    """The buckets are laid out once: a weight that was replaced by one of another shape, larger, smaller or of the same size,
+    raises as the copies between parameters and buckets do, and the buckets' other parts keep their values."""
+    from torchft_b200.local_sgd import _FlatBuckets
+    from torchft_b200.ops.outer_step import FusedOuterStep
+
+    params = [torch.nn.Parameter(torch.randn(s, device=DEV)) for s in ((6, 8), (16,))]
+    opt = torch.optim.SGD(params, lr=0.7, momentum=0.9)
+    backup, comm = _FlatBuckets(params, None, False), _FlatBuckets(params, None, False)
+    backup.copy_from_params()
+    comm.copy_from_params()
+    fused = FusedOuterStep.maybe_create(params, backup, comm, opt)
+    old = params[0].data
+    params[0].data = torch.randn(shape, device=DEV)
+    kept = [t.clone() for t in (comm.views[1], backup.views[0], backup.views[1])]
+    with pytest.raises(RuntimeError):
+        fused.compute_pseudogradients()
+    assert all(torch.equal(a, b) for a, b in zip((comm.views[1], backup.views[0], backup.views[1]), kept))
+    params[0].data = old
+    fused.compute_pseudogradients()
+    params[0].data = torch.randn(shape, device=DEV)
+    with pytest.raises(RuntimeError):
+        fused.apply_outer_update()
+
+
 @pytest.mark.parametrize("V", [8, 248, 256, 264, 2056, 32768, 32776, 65536, 65544, 128256, 262144, 262152])
 def test_cross_entropy_around_the_sizes_of_a_row_in_registers(V):
     """One warp, whole blocks, clusters of two to eight CTAs and the two-pass kernel beyond them; targets at both ends of the

@@ -174,24 +174,25 @@ class FusedOuterStep:
 
     def _table(self, key: Tuple[torch.dtype, torch.device]):
         """Addresses, bucket offsets and sizes of the parameters of one bucket, and the parameters that the kernels reach
-        only through their packed view (strided, or moved to another dtype or device since).  Built for every call:
-        nothing is kept by the address of a parameter."""
+        only through their packed view (strided, or given another dtype, device or shape since).  Built for every call:
+        nothing is kept by the address of a parameter.  Sizes are those of the bucket's views, which its memory is laid
+        out for; a parameter of another shape meets the copy to or from its view, which raises as it always did."""
         flat, (dtype, device) = self._comm.flat[key], key
         idxs = self._comm.groups[key]
         base, size = flat.data_ptr(), flat.element_size()
-        ptrs, offs, packed = [], [], []
+        ptrs, offs, sizes, packed = [], [], [], []
         for i in idxs:
             p, view = self._params[i], self._comm.views[i]
             assert view is not None
             at = view.data_ptr()
             offs.append((at - base) // size)
-            if p.is_contiguous() and p.dtype == dtype and p.device == device:
+            sizes.append(view.numel())
+            if p.is_contiguous() and p.dtype == dtype and p.device == device and p.shape == view.shape:
                 ptrs.append(p.data_ptr())
             else:
                 ptrs.append(at)
                 packed.append(i)
         n = len(idxs)
-        sizes = [self._params[i].numel() for i in idxs]
         return (ctypes.c_void_p * n)(*ptrs), (ctypes.c_int64 * n)(*offs), (ctypes.c_int64 * n)(*sizes), n, packed
 
     @staticmethod
