@@ -144,6 +144,55 @@ def test_gradient_buffers_under_saved_tensor_hooks(name, late):
     assert torch.equal(buffer, want)
 
 
+def at_odd_address(t):
+    flat = torch.full((t.numel() + 1,), float("nan"), device=t.device, dtype=t.dtype)
+    view = flat[1:].view(t.shape)
+    view.copy_(t.detach())
+    return view
+
+
+def in_wider_rows(t):
+    wide = torch.full((*t.shape[:-1], t.shape[-1] + 8), float("nan"), device=t.device, dtype=t.dtype)
+    wide[..., : t.shape[-1]] = t.detach()
+    return wide[..., : t.shape[-1]]
+
+
+@pytest.mark.parametrize("unpack", [at_odd_address, in_wider_rows, lambda t: t.detach().transpose(0, -1).contiguous().transpose(0, -1)],
+                         ids=["odd_address", "wider_rows", "transposed"])
+@pytest.mark.parametrize("name", CASES)
+def test_saved_tensors_of_another_layout(name, unpack):
+    """A hook may give back the values in any layout and at any address: the gradients are the same bit for bit."""
+    from torchft_b200.ops import attention as A
+    from torchft_b200.ops import functional as F
+
+    torch.manual_seed(0)
+    fn, _, inputs = CASES[name](F, A)
+    results = []
+    for hook in (lambda t: t.detach(), unpack):
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t, hook):
+            outs = fn(*inputs)
+        outs = outs if isinstance(outs, tuple) else (outs,)
+        torch.manual_seed(1)
+        results.append(torch.autograd.grad(outs, inputs, [unpack(torch.randn_like(o)) for o in outs]))
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("unpack", [lambda t: t.float() if t.dtype == torch.bfloat16 else t.double(), lambda t: t.detach()[..., :-1],
+                                    lambda t: t.cpu()], ids=["dtype", "size", "device"])
+@pytest.mark.parametrize("name", CASES)
+def test_saved_tensors_of_another_kind_are_refused(name, unpack):
+    from torchft_b200.ops import attention as A
+    from torchft_b200.ops import functional as F
+
+    fn, _, inputs = CASES[name](F, A)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+        out = fn(*inputs)
+    out = out[0] if isinstance(out, tuple) else out
+    with pytest.raises(RuntimeError, match="saved-tensor hook"):
+        torch.autograd.grad(out, inputs, torch.randn_like(out), allow_unused=True)
+
+
 def test_cross_entropy_matches_the_python_node():
     from torchft_b200.ops import functional as F
 

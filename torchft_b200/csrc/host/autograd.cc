@@ -95,7 +95,23 @@ bool has_main_grad(const Tensor& weight) {
 }
 bool fits_int(int64_t v) { return v >= 0 && v <= INT32_MAX; }
 
-Tensor dense(const Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
+// The kernels read dense rows in vectors of 16 bytes.
+bool aligned(const Tensor& t) { return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0; }
+Tensor dense(const Tensor& t) {
+  if (!t.is_contiguous()) return t.contiguous();
+  return aligned(t) ? t : t.clone();
+}
+
+// A saved tensor in the backward pass.  A hook may have unpacked another one than the forward pass looked at: of any strides
+// and at any address, which a copy mends, or of another kind, which is refused.
+bool is_operand(const Tensor& t, at::IntArrayRef sizes, const Tensor& grad, at::ScalarType type) {
+  return t.defined() && t.is_cuda() && t.device() == grad.device() && t.layout() == at::kStrided && t.scalar_type() == type &&
+         t.sizes() == sizes;
+}
+Tensor operand(const Tensor& t, at::IntArrayRef sizes, const Tensor& grad, at::ScalarType type = at::kBFloat16) {
+  TORCH_CHECK(is_operand(t, sizes, grad, type), "a saved-tensor hook unpacked another kind of tensor than the forward pass saved");
+  return dense(t);
+}
 
 // ------------------------------------------------------------------ linear
 // out [M, N] = op(a) op(b): a is [M, K], or [K, M] with a_mn; b is [N, K], or [K, N] with b_mn.  All dense.
@@ -121,16 +137,17 @@ struct Linear : public Function<Linear> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor &x = saved[0], &w = saved[1];
-    const int64_t N = w.size(0), K = w.size(1), M = x.numel() / K;
-    const Tensor dy = dense(grads[0]);
+    const Tensor dy = dense(grads[0]), weight = kept_weight(ctx);
+    const int64_t N = weight.size(0), K = weight.size(1), M = dy.numel() / N;
+    auto sizes = dy.sizes().vec();
+    sizes.back() = K;
+    const Tensor x = operand(saved[0], sizes, dy), w = operand(saved[1], {N, K}, dy);
     Tensor dx, dw;
     if (ctx->needs_input_grad(0)) {
       dx = at::empty_like(x);
       gemm(dy, w, dx, M, K, N, false, true);
     }
     if (ctx->needs_input_grad(1)) {
-      const Tensor weight = kept_weight(ctx);
       if (has_main_grad(weight)) {  // given to it since the forward pass
         py::gil_scoped_acquire gil;
         const py::object g = py::handle(linear_wgrad)(weight, dy.view({M, N}), x.view({M, K}));
@@ -164,10 +181,10 @@ bool norm_dim(int64_t dim) {
 }
 
 // (dx, dw) of y = rmsnorm(h) * w; dres is added to dx.
-std::pair<Tensor, Tensor> norm_backward(const Tensor& weight, const Tensor& grad_y, const Tensor& h, const Tensor& w,
-                                        const Tensor& rstd, const Tensor& grad_h) {
-  const int64_t dim = h.size(-1), rows = h.numel() / dim;
+std::pair<Tensor, Tensor> norm_backward(const Tensor& weight, const Tensor& grad_y, const variable_list& saved, const Tensor& grad_h) {
   const Tensor dy = dense(grad_y), dres = grad_h.defined() ? dense(grad_h) : grad_h;
+  const int64_t dim = dy.size(-1), rows = dy.numel() / dim;
+  const Tensor h = operand(saved[0], dy.sizes(), dy), w = operand(saved[1], {dim}, dy), rstd = operand(saved[2], {rows}, dy, at::kFloat);
   Tensor dx = at::empty_like(h), dw, out;
   bool accumulate = false;
   if (has_main_grad(weight)) {  // given to it since the forward pass
@@ -197,8 +214,7 @@ struct RMSNorm : public Function<RMSNorm> {
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const auto s = ctx->get_saved_variables();
-    auto [dx, dw] = norm_backward(kept_weight(ctx), grads[0], s[0], s[1], s[2], Tensor());
+    auto [dx, dw] = norm_backward(kept_weight(ctx), grads[0], ctx->get_saved_variables(), Tensor());
     return {dx, dw, Tensor()};
   }
 };
@@ -220,7 +236,7 @@ struct AddRMSNorm : public Function<AddRMSNorm> {
     // an output that took no part in the loss arrives as zeros, as in the Python node
     const Tensor dy = grads[0].defined() ? grads[0] : at::zeros_like(s[0]);
     const Tensor dh = grads[1].defined() ? grads[1] : at::zeros_like(s[0]);
-    auto [dx, dw] = norm_backward(kept_weight(ctx), dy, s[0], s[1], s[2], dh);
+    auto [dx, dw] = norm_backward(kept_weight(ctx), dy, s, dh);
     return {dx, dx, dw, Tensor()};
   }
 };
@@ -256,8 +272,11 @@ struct SwiGLU : public Function<SwiGLU> {
     return out;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
-    const Tensor gu = ctx->get_saved_variables()[0], dout = dense(grads[0]);
-    const int64_t F = gu.size(-1) / 2, rows = gu.numel() / (2 * F);
+    const Tensor dout = dense(grads[0]);
+    const int64_t F = dout.size(-1), rows = dout.numel() / F;
+    auto sizes = dout.sizes().vec();
+    sizes.back() = 2 * F;
+    const Tensor gu = operand(ctx->get_saved_variables()[0], sizes, dout);
     Tensor dgu = at::empty_like(gu);
     check(kernels.swiglu_bwd(gu.data_ptr(), dout.data_ptr(), dgu.data_ptr(), rows, F, stream()), "tft_swiglu_bwd");
     ++launched;
@@ -277,6 +296,9 @@ bool plain_heads(const Tensor& t) {  // [B, S, H, D], heads packed inside a toke
   return t.dim() == 4 && t.stride(3) == 1 && t.stride(2) == t.size(3) && t.stride(0) == t.stride(1) * t.size(1) &&
          t.stride(1) % 8 == 0 && fits_int(t.stride(1)) && t.stride(1) > 0;
 }
+Tensor heads_operand(const Tensor& t, at::IntArrayRef sizes, const Tensor& grad) {  // strided as it is where the kernel can
+  return is_operand(t, sizes, grad, at::kBFloat16) && plain_heads(t) && aligned(t) ? t : operand(t, sizes, grad);
+}
 struct Attention : public Function<Attention> {
   static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, double scale) {
     const int64_t B = q.size(0), S = q.size(1), Hq = q.size(2), D = q.size(3), Hkv = k.size(2);
@@ -291,9 +313,11 @@ struct Attention : public Function<Attention> {
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto s = ctx->get_saved_variables();
-    const Tensor &q = s[0], &k = s[1], &v = s[2], &o = s[3], &lse = s[4];
-    const int64_t B = q.size(0), S = q.size(1), Hq = q.size(2), D = q.size(3), Hkv = k.size(2);
     const Tensor d_o = dense(grads[0]);
+    const int64_t B = d_o.size(0), S = d_o.size(1), Hq = d_o.size(2), D = d_o.size(3), Hkv = s[1].size(2);
+    const Tensor q = heads_operand(s[0], {B, S, Hq, D}, d_o), k = heads_operand(s[1], {B, S, Hkv, D}, d_o);
+    const Tensor v = heads_operand(s[2], {B, S, Hkv, D}, d_o), o = operand(s[3], d_o.sizes(), d_o);
+    const Tensor lse = operand(s[4], {B, Hq, S}, d_o, at::kFloat);
     Tensor dq = at::empty({B, S, Hq, D}, q.options()), dk = at::empty({B, S, Hkv, D}, q.options());
     Tensor dv = at::empty({B, S, Hkv, D}, q.options()), delta = at::empty({B, Hq, S}, lse.options());
     check(kernels.attn_bwd(d_o.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(), delta.data_ptr(),
