@@ -417,6 +417,25 @@ def test_cross_entropy_around_the_sizes_of_a_row_in_registers(V):
     assert (work.grad[-1] == 0).all()
 
 
+@pytest.mark.parametrize("V,bad", [(1000, 8), (1000, 992), (32768, 64), (32768, 32760), (49152, 8), (49152, 16384), (49152, 49144)])
+def test_cross_entropy_keeps_nan(V, bad):
+    """Vectors, threads and whole rounds of nothing but NaN (beside -inf in one row) do not vanish: the loss and the row's
+    gradient are NaN, as for a NaN among finite logits, and the other rows keep their values."""
+    from torchft_b200.ops.functional import cross_entropy
+
+    torch.manual_seed(V)
+    logits, targets = bf16(4, V, scale=2.0), torch.tensor([1, V - 1, 2, V - 1], device=DEV)
+    clean = logits.clone()
+    cross_entropy(clean, targets)
+    logits[1, :bad] = float("nan")
+    logits[3, :bad] = float("-inf")
+    logits[3, bad // 2] = float("nan")
+    loss = cross_entropy(logits, targets)
+    assert torch.isnan(loss)
+    assert torch.isnan(logits[1]).all() and torch.isnan(logits[3]).all()
+    assert torch.equal(logits[::2], clean[::2])
+
+
 def test_adamw_of_many_tensors_equals_one_at_a_time():
     """Sizes around a vector and a block's chunk, an empty tensor, more tensors than one table holds: bit for bit the same."""
     from torchft_b200.ops.functional import adamw_multi_, adamw_step_

@@ -81,12 +81,14 @@ constexpr int XENT_THREADS = 512;
 constexpr int XENT_ROOM = XENT_THREADS * XENT_VECS;  // vectors of a row that one block takes
 
 struct MaxSum {
-  float m, s;  // maximum and sum of exp(x - m); an empty or all -inf part is (-inf, 0)
+  // Maximum and sum of exp(x - m); an empty or all -inf part is (-inf, 0).  The maximum passes over NaN and the sum does not:
+  // a part of nothing but NaN and -inf is (-inf, NaN), and makes the row's loss and gradient NaN.
+  float m, s;
 };
 __device__ __forceinline__ MaxSum combine(MaxSum a, MaxSum b) {
   MaxSum r;
   r.m = fmaxf(a.m, b.m);
-  r.s = (a.m == -INFINITY ? 0.f : a.s * __expf(a.m - r.m)) + (b.m == -INFINITY ? 0.f : b.s * __expf(b.m - r.m));
+  r.s = (a.m == -INFINITY ? a.s : a.s * __expf(a.m - r.m)) + (b.m == -INFINITY ? b.s : b.s * __expf(b.m - r.m));
   return r;
 }
 __device__ __forceinline__ MaxSum warp_combine(MaxSum v) {
@@ -204,16 +206,16 @@ xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ ta
 #pragma unroll
       for (int j = 0; j < 8; ++j) m = fmaxf(m, f[j]);
     }
-    if (m == -INFINITY) continue;  // nothing but -inf so far
+    const float base = m == -INFINITY ? 0.f : m;
     float s = 0.f;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       float f[8];
       ew_unpack8(v[u], f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) s += __expf(f[j] - m);
+      for (int j = 0; j < 8; ++j) s += __expf(f[j] - base);
     }
-    r.s = r.s * __expf(r.m - m) + s;
+    r.s = r.s * __expf(r.m - base) + s;
     r.m = m;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
