@@ -436,6 +436,26 @@ def test_cross_entropy_keeps_nan(V, bad):
     assert torch.equal(logits[::2], clean[::2])
 
 
+@pytest.mark.parametrize("shift", [0.0, 1e3, -1e6, 1e30, -3e38, torch.finfo(torch.bfloat16).min])
+@pytest.mark.parametrize("V", [1000, 32768, 49152])
+def test_cross_entropy_of_large_logits(V, shift):
+    """Loss and gradient depend on differences of logits, which bf16 values have exactly or with one rounding in fp32."""
+    from torchft_b200.ops.functional import cross_entropy
+
+    torch.manual_seed(V)
+    logits = torch.full((4, V), shift, device=DEV).to(torch.bfloat16) if abs(shift) > 1e6 else (torch.randn(4, V, device=DEV) * 4 + shift).to(torch.bfloat16)
+    targets = torch.tensor([0, 3, V // 2, V - 1], device=DEV)
+    x = logits.double().requires_grad_()
+    ref = torch.nn.functional.cross_entropy(x, targets)
+    ref.backward()
+    work = logits.clone().requires_grad_()
+    loss = cross_entropy(work, targets)
+    loss.backward()
+    # fp32 sums of exponentials good to 2e-6 each, and one rounding to bf16 of every gradient
+    assert abs(loss.item() - ref.item()) < 2e-5 * max(1.0, abs(ref.item()))
+    assert ((work.grad.double() - x.grad).abs() <= 2.0**-8 * x.grad.abs() + 1e-6).all()
+
+
 def test_adamw_of_many_tensors_equals_one_at_a_time():
     """Sizes around a vector and a block's chunk, an empty tensor, more tensors than one table holds: bit for bit the same."""
     from torchft_b200.ops.functional import adamw_multi_, adamw_step_

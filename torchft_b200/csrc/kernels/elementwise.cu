@@ -4,6 +4,8 @@
 // vector accesses, fp32 math.
 #include "common.cuh"
 
+#include <cfloat>
+
 namespace tft {
 
 __device__ __forceinline__ void ew_unpack8(const uint4& u, float (&f)[8]) {
@@ -75,20 +77,22 @@ __global__ void swiglu_bwd_kernel(const __nv_bfloat16* __restrict__ gu, const __
 // Two kernels.  Rows of up to 32768 columns stay in the registers of one block between the two passes, eight 16-byte
 // vectors a thread (xent_row_kernel).  Longer rows are read twice, the second time partly from L2 (xent_kernel): holding
 // them in the registers of a cluster of CTAs reads memory once but costs a cluster barrier a row, and took 311 to 430 us
-// where the two passes take 205 (2048 x 128256).
+// where the two passes took 205 (2048 x 128256).
 constexpr int XENT_VECS = 8;
 constexpr int XENT_THREADS = 512;
 constexpr int XENT_ROOM = XENT_THREADS * XENT_VECS;  // vectors of a row that one block takes
 
+// Maximum and sum of exp(x - m) of a part of a row.  The maximum starts at the lowest finite number, so that differences from it
+// are never those of two infinities: a part that is empty or all -inf has the sum 0.  The maximum passes over NaN and the sum
+// does not, so NaN makes the row's loss and gradient NaN; +inf does too, and a row of nothing but -inf.
 struct MaxSum {
-  // Maximum and sum of exp(x - m); an empty or all -inf part is (-inf, 0).  The maximum passes over NaN and the sum does not:
-  // a part of nothing but NaN and -inf is (-inf, NaN), and makes the row's loss and gradient NaN.
   float m, s;
 };
-__device__ __forceinline__ MaxSum combine(MaxSum a, MaxSum b) {
+__device__ __forceinline__ MaxSum empty_part() { return {-FLT_MAX, 0.f}; }
+__device__ __forceinline__ MaxSum combine(const MaxSum& a, const MaxSum& b) {
   MaxSum r;
   r.m = fmaxf(a.m, b.m);
-  r.s = (a.m == -INFINITY ? a.s : a.s * __expf(a.m - r.m)) + (b.m == -INFINITY ? b.s : b.s * __expf(b.m - r.m));
+  r.s = a.s * __expf(a.m - r.m) + b.s * __expf(b.m - r.m);
   return r;
 }
 __device__ __forceinline__ MaxSum warp_combine(MaxSum v) {
@@ -102,34 +106,42 @@ __device__ __forceinline__ MaxSum warp_combine(MaxSum v) {
   return v;
 }
 
-// The gradient of eight logits f of which element `here` (if below 8) is the target.  exp(f - lse) as one multiply-add and one
-// exp2; the target's own value, from which 1 is taken, without the rounding of lse * log2(e).
+// Eight softmax values times the gradient's scale: exp(f - m) * unit with the row's maximum m and unit = scale / s.  Differences
+// from the maximum are exact where they count, whatever the size of the logits.  From the log-sum-exp, which is rounded to the
+// size of the maximum, exp(f - lse) is off by up to 3 % at logits of 1e6, and lse * log2(e) overflows in rows of the type's
+// lowest value.  Two values at a time but for the exponential: both kernels are close to their issue rate here.
 constexpr float kLog2e = 1.4426950408889634f;
-__device__ __forceinline__ uint4 xent_grad(const uint4& u, float lse, float scale, unsigned here, float* loss) {
+__device__ __forceinline__ uint4 xent_grad(const uint4& u, float m, float unit) {
   float f[8];
   ew_unpack8(u, f);
-  float hot = 0.f;
-  if (here < 8u) {
+  const float2 less_m = make_float2(-m, -m), log2e = make_float2(kLog2e, kLog2e), units = make_float2(unit, unit);
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (here == j) hot = f[j];
-    *loss = lse - hot;
-    hot = (__expf(hot - lse) - 1.f) * scale;
-  }
-  const float c = lse * kLog2e;
-#pragma unroll
-  for (int j = 0; j < 8; ++j) f[j] = exp2f(fmaf(f[j], kLog2e, -c)) * scale;
-  if (here < 8u) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (here == j) f[j] = hot;
+  for (int j = 0; j < 8; j += 2) {
+    const float2 t = __fmul2_rn(__fadd2_rn(make_float2(f[j], f[j + 1]), less_m), log2e);
+    const float2 g = __fmul2_rn(make_float2(exp2f(t.x), exp2f(t.y)), units);
+    f[j] = g.x;
+    f[j + 1] = g.y;
   }
   return ew_pack8(f);
 }
 
+// The target's part, left to the thread that writes the target's vector: it reads the logit before the gradient goes over it
+// and takes 1 from the softmax there afterwards.  The vectors are stored as another type than the one element, so both
+// accesses are fenced off from them for the compiler.
+__device__ __forceinline__ float xent_target_logit(const __nv_bfloat16* at) {
+  const float hot = __bfloat162float(*at);
+  asm volatile("" ::: "memory");
+  return hot;
+}
+__device__ __forceinline__ void xent_target(__nv_bfloat16* at, float hot, const MaxSum& r, float unit, float* loss) {
+  asm volatile("" ::: "memory");
+  *loss = (r.m - hot) + __logf(r.s);
+  *at = __float2bfloat16((__expf(hot - r.m) - r.s) * unit);
+}
+
 // One block per row, as few threads as hold it: short rows then share an SM with more of their kind.  Bound by the launch
-// below a few thousand rows; 14.7 us for 26.6 with two passes at 2048 x 4096, 33.8 for 63.8 at 4096 x 8192, 7.9 for 12.8 at
-// 1024 x 1000, 265 for 281 at 8192 x 32000.
+// below a few thousand rows; 10.5 us for 26 with two passes at 2048 x 4096, 25.7 for 63.8 at 4096 x 8192, 5.8 for 12.6 at
+// 1024 x 1000, 213 for 282 at 8192 x 32000 (logits left in L2 by the call before where they fit).
 __global__ void __launch_bounds__(XENT_THREADS, 2)
 xent_row_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets, float* __restrict__ loss, int V,
                 int ld, float grad_scale, long long ignore_index) {
@@ -138,11 +150,14 @@ xent_row_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict_
   const int n = V / 8, step = blockDim.x;
   uint4* z = reinterpret_cast<uint4*>(logits + row * ld) + threadIdx.x;
   const long long tgt = targets[row];
+  const bool ignored = tgt == ignore_index || tgt < 0 || tgt >= V;
+  const bool mine = !ignored && static_cast<int>(tgt) / 8 % step == static_cast<int>(threadIdx.x);
+  const float hot = mine ? xent_target_logit(logits + row * ld + tgt) : 0.f;
   uint4 v[XENT_VECS];
 #pragma unroll
   for (int k = 0; k < XENT_VECS; ++k)
     v[k] = static_cast<int>(threadIdx.x) + k * step < n ? z[k * step] : make_uint4(0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u, 0xFF80FF80u);  // -inf
-  MaxSum r = {-INFINITY, 0.f};
+  MaxSum r = empty_part();
 #pragma unroll
   for (int k = 0; k < XENT_VECS; ++k) {
     float f[8];
@@ -150,37 +165,34 @@ xent_row_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict_
 #pragma unroll
     for (int j = 0; j < 8; ++j) r.m = fmaxf(r.m, f[j]);
   }
-  const float base = r.m == -INFINITY ? 0.f : r.m;
 #pragma unroll
   for (int k = 0; k < XENT_VECS; ++k) {
     float f[8];
     ew_unpack8(v[k], f);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) r.s += __expf(f[j] - base);
+    for (int j = 0; j < 8; ++j) r.s += __expf(f[j] - r.m);
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   r = warp_combine(r);
   if (warps > 1) {
     if (lane == 0) part[warp] = r;
     __syncthreads();
-    r = warp_combine(lane < warps ? part[lane] : MaxSum{-INFINITY, 0.f});
+    r = warp_combine(lane < warps ? part[lane] : empty_part());
   }
-  const float lse = r.m + __logf(r.s);
-  const bool ignored = tgt == ignore_index || tgt < 0 || tgt >= V;
-  if (ignored && threadIdx.x == 0) loss[row] = 0.f;
-  const float scale = ignored ? 0.f : grad_scale;
-  // place of the target among this thread's vectors: element hot % 8 of vector hot / 8 counted from its first
-  const int hot = ignored ? -1 : static_cast<int>(tgt) - static_cast<int>(threadIdx.x) * 8;
+  const float unit = (ignored ? 0.f : grad_scale) / r.s;
 #pragma unroll
   for (int k = 0; k < XENT_VECS; ++k, z += step) {
     if (static_cast<int>(threadIdx.x) + k * step >= n) break;
-    *z = xent_grad(v[k], lse, scale, static_cast<unsigned>(hot - k * step * 8), loss + row);
+    *z = xent_grad(v[k], r.m, unit);
   }
+  if (mine) xent_target(logits + row * ld + tgt, hot, r, unit, loss + row);
+  if (ignored && threadIdx.x == 0) loss[row] = 0.f;
 }
 
 // Pass 1: online maximum and sum of exponentials.  Pass 2 (in place): the gradient.  Two vectors a thread and round in flight,
-// two blocks of 1024 per SM: 205 us at 2048 x 128256 (158 for one read and one write at the copy bandwidth), 241 with one.
-// Four vectors and half the threads: 215; one block per SM: 214.
+// two blocks of 1024 per SM: 200 us at 2048 x 128256 (158 for one read and one write at the copy bandwidth), 241 with one.
+// Four vectors and half the threads, or one block per SM, cost 5 % more.  With the target's element picked out inside the
+// second loop the kernel spills at its 32 registers: 213.
 constexpr int XENT_LONG_THREADS = 1024;
 constexpr int XENT_LONG_VECS = 2;
 __global__ void __launch_bounds__(XENT_LONG_THREADS, 2)
@@ -192,7 +204,10 @@ xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ ta
   const int n = V / 8;
   uint4* z = reinterpret_cast<uint4*>(logits + row * ld);
   const long long tgt = targets[row];
-  MaxSum r = {-INFINITY, 0.f};
+  const bool ignored = tgt == ignore_index || tgt < 0 || tgt >= V;
+  const bool mine = !ignored && static_cast<int>(tgt) / 8 % STEP == static_cast<int>(threadIdx.x);
+  const float hot = mine ? xent_target_logit(logits + row * ld + tgt) : 0.f;
+  MaxSum r = empty_part();
   for (int i0 = threadIdx.x; i0 < n; i0 += U * STEP) {
     uint4 v[U];
 #pragma unroll
@@ -206,16 +221,15 @@ xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ ta
 #pragma unroll
       for (int j = 0; j < 8; ++j) m = fmaxf(m, f[j]);
     }
-    const float base = m == -INFINITY ? 0.f : m;
     float s = 0.f;
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       float f[8];
       ew_unpack8(v[u], f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) s += __expf(f[j] - base);
+      for (int j = 0; j < 8; ++j) s += __expf(f[j] - m);
     }
-    r.s = r.s * __expf(r.m - base) + s;
+    r.s = r.s * __expf(r.m - m) + s;
     r.m = m;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -223,11 +237,7 @@ xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ ta
   if (lane == 0) part[warp] = r;
   __syncthreads();
   r = warp_combine(part[lane]);
-  const float lse = r.m + __logf(r.s);
-  const bool ignored = tgt == ignore_index || tgt < 0 || tgt >= V;
-  if (ignored && threadIdx.x == 0) loss[row] = 0.f;
-  const float scale = ignored ? 0.f : grad_scale;
-  const int hot = ignored ? -1 : static_cast<int>(tgt);
+  const float unit = (ignored ? 0.f : grad_scale) / r.s;
   for (int i0 = threadIdx.x; i0 < n; i0 += U * STEP) {
     uint4 v[U];
 #pragma unroll
@@ -236,9 +246,11 @@ xent_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ ta
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const int i = i0 + u * STEP;
-      if (i < n) z[i] = xent_grad(v[u], lse, scale, static_cast<unsigned>(hot - i * 8), loss + row);
+      if (i < n) z[i] = xent_grad(v[u], r.m, unit);
     }
   }
+  if (mine) xent_target(logits + row * ld + tgt, hot, r, unit, loss + row);
+  if (ignored && threadIdx.x == 0) loss[row] = 0.f;
 }
 
 // ------------------------------------------------------------------ embedding
