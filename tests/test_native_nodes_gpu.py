@@ -1,5 +1,7 @@
 """The native autograd nodes give the values of the Python nodes, and leave to those every call that is not plain."""
 
+import ctypes
+
 import pytest
 import torch
 
@@ -191,6 +193,28 @@ def test_saved_tensors_of_another_kind_are_refused(name, unpack):
     out = out[0] if isinstance(out, tuple) else out
     with pytest.raises(RuntimeError, match="saved-tensor hook"):
         torch.autograd.grad(out, inputs, torch.randn_like(out), allow_unused=True)
+
+
+def test_the_interpreter_lock_is_free_during_launches():
+    """In place of every kernel's entry stands the question whether this thread holds the lock: 1 is an error, 0 success."""
+    from torchft_b200.ops import _lib, _native
+    from torchft_b200.ops import attention as A
+    from torchft_b200.ops import functional as F
+
+    entries = {name: ctypes.cast(getattr(_lib.lib(), name), ctypes.c_void_p).value for name in _native._ENTRIES}
+    others = (_lib.KernelError, _native._status_address, F._weight_gradient, F._main_grad_target)
+    holds = ctypes.cast(ctypes.pythonapi.PyGILState_Check, ctypes.c_void_p).value
+    sizes = ("tft_gemm2_workspace", "tft_rmsnorm_bwd_parts")
+    m = _native.module()
+    calls = [(fn, inputs) for fn, _, inputs in (case(F, A) for case in CASES.values())]
+    calls.append((F.cross_entropy, [leaf(33, 1000), torch.randint(1000, (33,), device=DEV)]))
+    m.setup({name: at if name in sizes else holds for name, at in entries.items()}, *others)
+    try:
+        for fn, inputs in calls:
+            out = fn(*inputs)
+            (out[0] if isinstance(out, tuple) else out).sum().backward()
+    finally:
+        m.setup(entries, *others)
 
 
 def test_cross_entropy_matches_the_python_node():

@@ -93,6 +93,13 @@ bool has_main_grad(const Tensor& weight) {
   py::gil_scoped_acquire gil;
   return has_main_grad(py::reinterpret_steal<py::object>(THPVariable_Wrap(weight)));
 }
+// Runs a node's forward pass as torch runs its own operators and ctypes its calls: without the interpreter lock.  An allocation
+// or a launch may block behind a collective that hangs, and the Python thread that aborts it has to run.
+template <typename Apply>
+auto unlocked(Apply apply) {
+  py::gil_scoped_release no_gil;
+  return apply();
+}
 bool fits_int(int64_t v) { return v >= 0 && v <= INT32_MAX; }
 
 // The kernels read dense rows in vectors of 16 bytes.
@@ -169,7 +176,7 @@ py::object linear(py::handle hx, py::handle hw) {
       x.get_device() != w.get_device())
     return py::none();
   if (has_main_grad(hw) || PyObject_HasAttrString(hw.ptr(), "gather_comm")) return py::none();
-  return py::cast(Linear::apply(x, w));
+  return py::cast(unlocked([&] { return Linear::apply(x, w); }));
 }
 
 // ------------------------------------------------------------------ RMSNorm
@@ -249,13 +256,14 @@ bool plain_norm(py::handle hx, py::handle hw) {
 }
 py::object rmsnorm(py::handle hx, py::handle hw, double eps) {
   if (!plain_norm(hx, hw)) return py::none();
-  return py::cast(RMSNorm::apply(THPVariable_Unpack(hx.ptr()), THPVariable_Unpack(hw.ptr()), eps));
+  const Tensor &x = THPVariable_Unpack(hx.ptr()), &w = THPVariable_Unpack(hw.ptr());
+  return py::cast(unlocked([&] { return RMSNorm::apply(x, w, eps); }));
 }
 py::object add_rmsnorm(py::handle hx, py::handle hr, py::handle hw, double eps) {
   if (!plain_norm(hx, hw) || !plain(hr)) return py::none();
-  const Tensor &x = THPVariable_Unpack(hx.ptr()), &res = THPVariable_Unpack(hr.ptr());
+  const Tensor &x = THPVariable_Unpack(hx.ptr()), &res = THPVariable_Unpack(hr.ptr()), &w = THPVariable_Unpack(hw.ptr());
   if (!res.is_contiguous() || res.sizes() != x.sizes() || res.get_device() != x.get_device()) return py::none();
-  const variable_list out = AddRMSNorm::apply(x, res, THPVariable_Unpack(hw.ptr()), eps);
+  const variable_list out = unlocked([&] { return AddRMSNorm::apply(x, res, w, eps); });
   return py::make_tuple(out[0], out[1]);
 }
 
@@ -287,7 +295,7 @@ py::object swiglu(py::handle h) {
   if (!plain(h) || !plain_context()) return py::none();
   const Tensor& gu = THPVariable_Unpack(h.ptr());
   if (gu.dim() < 1 || !gu.is_contiguous() || gu.size(-1) % 16 || !fits_int(gu.size(-1))) return py::none();
-  return py::cast(SwiGLU::apply(gu));
+  return py::cast(unlocked([&] { return SwiGLU::apply(gu); }));
 }
 
 // ------------------------------------------------------------------ attention
@@ -335,7 +343,7 @@ py::object attention(py::handle hq, py::handle hk, py::handle hv, double scale) 
       q.size(1) != k.size(1) || q.size(3) != k.size(3) || (q.size(3) != 64 && q.size(3) != 128) || q.size(2) % k.size(2) || !(scale > 0) ||
       !fits_int(q.size(1)) || !fits_int(q.size(0)) || q.get_device() != k.get_device() || q.get_device() != v.get_device())
     return py::none();
-  return py::cast(Attention::apply(q, k, v, scale));
+  return py::cast(unlocked([&] { return Attention::apply(q, k, v, scale); }));
 }
 
 // ------------------------------------------------------------------ cross entropy (mean over all rows)
@@ -358,7 +366,7 @@ py::object cross_entropy(py::handle hl, py::handle ht) {
       !fits_int(logits.numel() / logits.size(-1)) || targets.numel() != logits.numel() / logits.size(-1) ||
       logits.get_device() != targets.get_device())
     return py::none();
-  return py::cast(CrossEntropy::apply(logits, targets));
+  return py::cast(unlocked([&] { return CrossEntropy::apply(logits, targets); }));
 }
 
 template <typename F>
