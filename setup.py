@@ -1,7 +1,9 @@
 """Builds the native parts in-tree (nvcc for sm_100a, g++ for the control plane) before packaging.
 
 ``python setup.py build_ext --inplace`` and ``pip install -e .`` both end up in
-``torchft_b200.utils.build.build_all``; the shared objects live inside the package directory.
+``torchft_b200.utils.build``; the shared objects live inside the package directory.  The native autograd nodes are built
+against the torch that is installed, so the package has to be built without isolation:
+``pip install --no-build-isolation -e .``.
 """
 
 import os
@@ -17,7 +19,14 @@ sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
 def _build_native() -> None:
     from torchft_b200.utils import build
 
-    build.build_all()
+    obstacle = build.autograd_obstacle()
+    if obstacle is None:
+        build.build_all()
+        return
+    # everything but the one part that needs torch's headers; using that part later raises and says what to run
+    build.build_control()
+    build.build_kernels()
+    print(f"native autograd nodes not built: {obstacle}", file=sys.stderr)
 
 
 class BuildNative(build_ext):

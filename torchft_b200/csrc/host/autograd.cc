@@ -395,6 +395,7 @@ void setup(const py::dict& entries, py::object error, py::object status, py::obj
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.doc() = "Autograd nodes of the plain cases; every function returns None for a call that the Python node has to take.";
+  m.attr("torch_mark") = TFT_TORCH_MARK;  // which torch this was built against (utils/build.py)
   m.def("setup", &setup);
   m.def("launches", [] { return launched.load(); });
   m.def("linear", &linear);

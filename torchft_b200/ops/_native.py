@@ -40,6 +40,10 @@ def _load():
             handle = _lib.lib()
             entries = {name: ctypes.cast(getattr(handle, name), ctypes.c_void_p).value for name in _ENTRIES}
             loaded = importlib.import_module("torchft_b200._autograd")
+            mark = getattr(loaded, "torch_mark", "built against an unknown torch;")
+            if mark != _build._torch_mark(torch.__version__):
+                raise _lib.KernelError(f"{path} was {mark[:-1]}, but torch {torch.__version__} runs: rebuild it with "
+                                       "`python -m torchft_b200.utils.build`")
             loaded.setup(entries, _lib.KernelError, _status_address, functional._weight_gradient, functional._main_grad_target)
             _lib.add_launch_counter(loaded.launches)
             _module = loaded

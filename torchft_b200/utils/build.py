@@ -21,7 +21,7 @@ import sys
 import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
-from typing import List
+from typing import List, Optional
 
 PKG = Path(__file__).resolve().parent.parent
 KERNEL_SRC = PKG / "csrc" / "kernels"
@@ -113,23 +113,51 @@ def _host_cxx() -> str:
     return os.environ.get("TFT_CXX") or ("/usr/bin/g++" if Path("/usr/bin/g++").exists() else os.environ.get("CXX", "g++"))
 
 
-def build_autograd(force: bool = False) -> Path:
-    """Builds the native autograd nodes against the installed torch."""
+def _torch_mark(version: str) -> str:
+    """What the module carries inside itself about the torch that it was built against."""
+    return f"built against torch {version};"
+
+
+def autograd_obstacle() -> Optional[str]:
+    """Why the native autograd nodes cannot be built in this environment, or ``None``."""
+    try:
+        import torch
+    except ImportError:
+        return ("torch is not installed here.  A package build in an isolated environment does not see the torch it will run with: "
+                "install with `pip install --no-build-isolation`, or run `python -m torchft_b200.utils.build` afterwards")
+    if torch.version.cuda is None:
+        return f"torch {torch.__version__} was built without CUDA"
+    return None
+
+
+def autograd_module_current() -> bool:
+    """Whether the module is there, newer than its source and built against the torch that is installed.  The file itself
+    says against which: the times of torch's files do not, since installers keep those of the archive or of a cache."""
     import torch
 
-    src = HOST_SRC / "autograd.cc"
     out = autograd_module_path()
-    torch_dir = Path(torch.__file__).parent
-    # rebuilt for another torch as well: the module follows its C++ interface
-    newest = max(_newest([src]), (torch_dir / "version.py").stat().st_mtime)
-    if not force and out.exists() and out.stat().st_mtime >= newest:
+    return (out.exists() and out.stat().st_mtime >= _newest([HOST_SRC / "autograd.cc"])
+            and _torch_mark(torch.__version__).encode() in out.read_bytes())
+
+
+def build_autograd(force: bool = False) -> Path:
+    """Builds the native autograd nodes against the installed torch."""
+    obstacle = autograd_obstacle()
+    if obstacle is not None:
+        raise RuntimeError(f"the native autograd nodes cannot be built: {obstacle}")
+    import torch
+
+    out = autograd_module_path()
+    if not force and autograd_module_current():
         return out
+    torch_dir = Path(torch.__file__).parent
     cuda_home = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
     cmd = [_host_cxx(), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_EXTENSION_NAME=_autograd",
+           f'-DTFT_TORCH_MARK="{_torch_mark(torch.__version__)}"',
            "-DTORCH_API_INCLUDE_EXTENSION_H", "-I", str(torch_dir / "include"),
            "-I", str(torch_dir / "include" / "torch" / "csrc" / "api" / "include"), "-I", str(cuda_home / "include"),
-           "-I", sysconfig.get_paths()["include"], str(src), "-o", str(out), "-L", str(torch_dir / "lib"),
+           "-I", sysconfig.get_paths()["include"], str(HOST_SRC / "autograd.cc"), "-o", str(out), "-L", str(torch_dir / "lib"),
            "-ltorch", "-ltorch_cpu", "-ltorch_python", "-lc10", "-lc10_cuda"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
