@@ -484,6 +484,28 @@ def test_adamw_of_many_tensors_equals_one_at_a_time():
     assert ((p - want).abs() <= 2.0**-8 * want.abs() + 1e-6).all()
 
 
+def test_adamw_of_parameters_that_share_memory():
+    """One parameter listed twice, two that are the same memory, two that overlap: the updates follow one another, as one call
+    for each would have them."""
+    from torchft_b200.ops.functional import adamw_multi_, adamw_step_
+
+    torch.manual_seed(0)
+    kw = dict(lr=1e-2, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, step=3)
+    base = bf16(200_000)
+    before = base.clone()
+    spans = [(0, 100_000), (100_000, 150_000), (0, 100_000), (0, 100_000), (99_992, 100_008), (150_000, 200_000)]
+    gs = [bf16(b - a) for a, b in spans]
+    ms, vs = [torch.randn(b - a, device=DEV) for a, b in spans], [torch.rand(b - a, device=DEV) for a, b in spans]
+    ms[2], vs[2] = ms[0], vs[0]  # the first one again
+    want_m, want_v = [m.clone() for m in ms], [v.clone() for v in vs]
+    want_m[2], want_v[2] = want_m[0], want_v[0]
+    adamw_multi_([base[a:b] for a, b in spans], gs, ms, vs, **kw)
+    for (a, b), g, m, v in zip(spans, gs, want_m, want_v):
+        adamw_step_(before[a:b], g, m, v, **kw)
+    assert torch.equal(base, before)
+    assert all(torch.equal(x, y) for x, y in zip(ms + vs, want_m + want_v))
+
+
 @pytest.mark.parametrize("a_k,b_k", [(True, True), (True, False), (False, False)])
 @pytest.mark.parametrize("shape", [(1, 8, 2048), (256, 256, 2045 * 8), (257, 264, 2112), (1013, 2048, 5464), (300, 4600, 4104), (9471, 8, 2056)])
 def test_gemm_with_a_divided_contraction(shape, a_k, b_k):

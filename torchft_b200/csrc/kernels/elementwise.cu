@@ -294,7 +294,8 @@ __device__ __forceinline__ int table_find(const int* first, int count, int c) {
 // ------------------------------------------------------------------ AdamW
 // p (bf16) updated in place from g (bf16) with fp32 moments; decoupled weight decay.
 // bc1 = 1 - beta1^t, bc2 = 1 - beta2^t.  grad_scale multiplies g first (1/accumulation steps).
-// One launch for up to kAdamMax tensors, whose addresses travel as an argument; a block handles one chunk of one tensor.
+// One launch for up to kAdamMax tensors without memory in common, whose addresses travel as an argument; a block handles one
+// chunk of one tensor.
 // Bound by HBM: 22 bytes a parameter.  The launch for every tensor that this replaces cost a model of small tensors more
 // than the update (see tft_adamw_multi).
 constexpr int kAdamMax = 80;
@@ -616,8 +617,18 @@ TFT_API int tft_adamw_multi(void* const* p, const void* const* g, float* const* 
     AdamTable tab;
     tab.count = 0;
     tab.first[0] = 0;
+    uintptr_t low = UINTPTR_MAX, high = 0;  // all parameters of the table lie between
     for (; i < count && tab.count < kAdamMax; ++i) {
       if (n[i] <= 0) continue;
+      // Parameters that share memory (tied weights, one listed twice) take their updates one after the other: the next launch
+      const uintptr_t begin = reinterpret_cast<uintptr_t>(p[i]), end = begin + static_cast<uintptr_t>(n[i]) * sizeof(__nv_bfloat16);
+      bool shared = false;
+      if (begin < high && low < end)
+        for (int k = 0; k < tab.count && !shared; ++k)
+          shared = begin < reinterpret_cast<uintptr_t>(tab.p[k] + tab.n[k]) && reinterpret_cast<uintptr_t>(tab.p[k]) < end;
+      if (shared) break;
+      low = begin < low ? begin : low;
+      high = end > high ? end : high;
       const int k = tab.count++;
       tab.p[k] = static_cast<__nv_bfloat16*>(p[i]);
       tab.g[k] = static_cast<const __nv_bfloat16*>(g[i]);
