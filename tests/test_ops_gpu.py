@@ -390,10 +390,11 @@ def test_outer_step_refuses_a_parameter_of_another_shape(shape):
         fused.apply_outer_update()
 
 
-@pytest.mark.parametrize("V", [8, 248, 256, 264, 2056, 32768, 32776, 65536, 65544, 128256, 262144, 262152])
+@pytest.mark.parametrize("V", [8, 248, 256, 264, 2056, 32768, 32776, 49144, 49152, 49160, 65536, 65544, 128256, 262144, 262152])
 def test_cross_entropy_around_the_sizes_of_a_row_in_registers(V):
-    """One warp, whole blocks, clusters of two to eight CTAs and the two-pass kernel beyond them; targets at both ends of the
-    row and around the borders of the parts, logits of -inf (also a whole first vector of them) and an ignored row."""
+    """Rows held in the registers of one warp and of blocks of up to 512 threads (up to 32768 columns), and rows read twice, in
+    rounds of 16384 columns; targets at both ends of the row and around its halves and quarters, logits of -inf (also a whole
+    first vector of them) and an ignored row."""
     from torchft_b200.ops.functional import cross_entropy
 
     torch.manual_seed(V)

@@ -161,14 +161,6 @@ __device__ __forceinline__ void store_acc(uint32_t taddr, __nv_bfloat16* dst, lo
   }
 }
 
-// Streaming multiprocessors of the current device (the attribute query takes tens of nanoseconds: nothing is kept).
-inline int sm_count() {
-  int dev = 0, sms = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
-    sms = 148;
-  return sms;
-}
-
 // 4-D tensor map over x[batch, seq, heads, HD] (token stride `ld` elements) with boxes of
 // {64, 1, 128, 1}.
 inline bool make_attn_tensormap(CUtensorMap* out, const void* ptr, int hd, int heads, int seq, int batch,

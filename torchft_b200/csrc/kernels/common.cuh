@@ -139,27 +139,15 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint6
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem desc]   (A operand read from tensor memory)
-__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc,
-                                             uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
-      "}\n" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // mbarrier arrives once every previously issued tcgen05.mma of this thread retired.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");
 }
-// The same three for a warp that stays converged: every lane runs the issuing code and `leader` (elect_one) picks the lane
-// that issues.  tcgen05.mma takes its descriptors from uniform registers; inside a branch that only one lane enters the
-// compiler moves each of them there anew for every instruction, which costs more than a 128 x 128 x 16 product takes
-// (64 cycles; 67 to 110 were measured between instructions, whatever their width).  dQ: 196 -> 168 us, forward: 146 -> 131
+// The same two for a warp that stays converged, and a product whose A operand is read from tensor memory (_ts): every lane runs
+// the issuing code and `leader` (elect_one) picks the lane that issues.  Issued inside a branch that one lane enters, 67 to 110
+// cycles were measured between instructions, whatever their width, where a 128 x 128 x 16 product takes 64; presumably the
+// operands that the instruction wants uniform are not so there.  dQ: 196 -> 168 us, forward: 146 -> 131
 // (S 4096, 32/8 heads of 128); CTA-pair GEMM 4096 x 28672 x 4096 forward: 659 -> 647 us, 1013 x 5464 x 2048: 29.6 -> 26.3.
 __device__ __forceinline__ void umma_bf16_elect(uint32_t leader, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
                                                 uint32_t idesc, uint32_t accumulate) {
@@ -279,6 +267,14 @@ __device__ __forceinline__ void exchange_quad(uint4 (&u)[4]) {
       if (upper) u[lo] = give; else u[hi] = give;
     }
   }
+}
+
+// Streaming multiprocessors of the current device (the attribute query takes tens of nanoseconds: nothing is kept).
+inline int sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1)
+    sms = 148;
+  return sms;
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {

@@ -145,8 +145,8 @@ __host__ __device__ inline Schedule make_schedule(int M, int N, int K, int pairs
 }
 
 // k-blocks per part of the contraction.  Divided where the tiles leave at least half of the pairs idle and the contraction is
-// long enough to pay for the second kernel (4 us, against 0.4 to 0.5 us a k-block); a part keeps eight k-blocks (more than
-// the pipeline holds) and the units still fit one wave.  1013 x 2048 x 5464 (32 tiles, input gradient):
+// long enough to pay for the second kernel (4 us, against 0.4 to 0.5 us a k-block); a part has at least
+// eight k-blocks (more than the pipeline holds; the last part, what is left) and the units still fit one wave.  1013 x 2048 x 5464 (32 tiles, input gradient):
 // 21.6 + 3.7 us for 33.6; 256 x 1024 x 4096 (4 tiles): 9.4 + 3.4 for 38.
 __host__ inline int kblocks_per_part(int M, int N, int K, int pairs) {
   const int kblocks = (K + BK - 1) / BK;

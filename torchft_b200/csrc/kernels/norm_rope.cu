@@ -100,6 +100,8 @@ __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __
 // Bound by memory (three reads and a write of [rows, dim]) and, with few rows per block in flight, by its latency: rows of up
 // to 4096 elements (VPT 1) fetch the next row ahead.  4096 x 4096 with residual gradient: 25.6 us for 36.8, and 3.7 for 7.4 in the
 // reduction behind it (half the partial rows, four loads in flight); both operands of the case are partly in L2.
+// Blocks have at most 512 threads.  The bound of 768 for VPT 2 stands for its registers: 80, where 512 would let it take 110 and
+// leave an SM one block of 320 to 384 threads instead of two.
 template <int VPT>
 __global__ void __launch_bounds__(VPT == 2 ? 768 : 512, VPT == 1 ? 2 : 1)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
@@ -261,8 +263,12 @@ static int norm_config(int dim, int* threads) {
 
 using namespace tft;
 
-// Number of dw partial rows the backward writes (size the scratch as parts * dim floats).
-TFT_API int tft_rmsnorm_bwd_parts(int rows) { return rows < 592 ? rows : 592; }
+// The most dw partial rows that the backward writes, whatever the width (size the scratch as parts * dim floats): four blocks
+// per SM, each with a partial sum of its own.
+TFT_API int tft_rmsnorm_bwd_parts(int rows) {
+  const int most = 4 * sm_count();
+  return rows < most ? rows : most;
+}
 
 TFT_API int tft_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* h_out, float* rstd,
                             int rows, int dim, float eps, cudaStream_t stream) {
@@ -292,7 +298,7 @@ TFT_API int tft_rmsnorm_bwd(const void* dy, const void* x, const void* w, const 
   if (!vpt || rows <= 0) return static_cast<int>(cudaErrorInvalidValue);
   // Rows that are fetched ahead: one wave (blocks of more than 256 threads fit an SM twice, of up to 256 four times), and no
   // more rows of partial sums than that.
-  const int most = tft_rmsnorm_bwd_parts(rows), wave = vpt == 1 && threads > 256 ? 296 : 592;
+  const int most = tft_rmsnorm_bwd_parts(rows), wave = (vpt == 1 && threads > 256 ? 2 : 4) * sm_count();
   const int parts = most < wave ? most : wave;
   auto DY = static_cast<const __nv_bfloat16*>(dy);
   auto X = static_cast<const __nv_bfloat16*>(x);
