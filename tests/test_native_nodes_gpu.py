@@ -195,6 +195,44 @@ def test_saved_tensors_of_another_kind_are_refused(name, unpack):
         torch.autograd.grad(out, inputs, torch.randn_like(out), allow_unused=True)
 
 
+def test_checkpointed_plain_layers():
+    """Recomputation stops early by an exception out of a hook, in the middle of a native node's forward pass."""
+    from torch.utils.checkpoint import checkpoint
+
+    from torchft_b200.ops import functional as F
+
+    torch.manual_seed(0)
+    x, n, w13, w2 = leaf(16, 256), leaf(256), leaf(128, 256, scale=0.1), leaf(256, 64, scale=0.1)
+
+    def block(x_):
+        return F.linear(F.swiglu(F.linear(F.rmsnorm(x_, n), w13)), w2)
+
+    dy = torch.randn(16, 256, device=DEV).to(torch.bfloat16)
+    want = torch.autograd.grad(block(x), (x, n, w13, w2), dy)
+    got = torch.autograd.grad(checkpoint(block, x, use_reentrant=False), (x, n, w13, w2), dy)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("name", CASES)
+def test_exceptions_of_hooks_keep_their_type(name):
+    from torchft_b200.ops import attention as A
+    from torchft_b200.ops import functional as F
+
+    class Unwilling(Exception):
+        pass
+
+    def refuse(t):
+        raise Unwilling("hook")
+
+    fn, _, inputs = CASES[name](F, A)
+    with torch.autograd.graph.saved_tensors_hooks(refuse, lambda t: t), pytest.raises(Unwilling):
+        fn(*inputs)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, refuse):
+        out = fn(*inputs)
+    with pytest.raises(Unwilling):
+        (out[0] if isinstance(out, tuple) else out).sum().backward()
+
+
 def test_the_interpreter_lock_is_free_during_launches():
     """In place of every kernel's entry stands the question whether this thread holds the lock: 1 is an error, 0 success."""
     from torchft_b200.ops import _lib, _native
