@@ -624,7 +624,7 @@ attn_dkdv_tmem_kernel(const __grid_constant__ CUtensorMap tq, const __grid_const
 //
 //   dV(t) half 0 | dK(t-1) half 1 | dP(t) half 1 | dV(t) half 1 | S(t+2) | dK(t) half 0 | dP(t+1) half 0
 //
-// Two sequences of 2048, 32/8 heads of 64, beside attn_dkdv_split_kernel on the same box: 88 us for 134; with the groups
+// Two sequences of 2048, 32/8 heads of 64, beside attn_dkdv_split_kernel on the same GPU: 88 us for 134; with the groups
 // taking turns on whole items (one dP region makes dS, dK and the next dP a chain) 90 for 128; with sixteen warps on one item
 // 101 for 138; with eight warps, before the MMA warp stayed converged, 104 for 129.
 struct DkvHalves {
