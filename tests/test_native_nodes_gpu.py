@@ -146,6 +146,23 @@ def test_gradient_buffers_under_saved_tensor_hooks(name, late):
     assert torch.equal(buffer, want)
 
 
+@pytest.mark.parametrize("shape", [(16, 64), (64, 64), (32, 128), (32, 32), (2048,)])
+def test_a_weight_replaced_between_the_passes_is_refused(shape):
+    """The sizes of the backward products come from the gradient and every operand is held against them."""
+    from torchft_b200.ops import functional as F
+
+    x, w = leaf(16, 64), leaf(32, 64)
+    y = F.linear(x, w)
+    w.data = torch.zeros(shape, device=DEV, dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError):
+        y.backward(torch.ones_like(y))
+    n = leaf(256)
+    y = F.rmsnorm(leaf(4, 256), n)
+    n.data = torch.ones(512, device=DEV, dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError):
+        y.backward(torch.ones_like(y))
+
+
 def at_odd_address(t):
     flat = torch.full((t.numel() + 1,), float("nan"), device=t.device, dtype=t.dtype)
     view = flat[1:].view(t.shape)

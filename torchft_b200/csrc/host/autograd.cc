@@ -117,7 +117,7 @@ bool is_operand(const Tensor& t, at::IntArrayRef sizes, const Tensor& grad, at::
          t.sizes() == sizes;
 }
 Tensor operand(const Tensor& t, at::IntArrayRef sizes, const Tensor& grad, at::ScalarType type = at::kBFloat16) {
-  TORCH_CHECK(is_operand(t, sizes, grad, type), "a saved-tensor hook unpacked another kind of tensor than the forward pass saved");
+  TORCH_CHECK(is_operand(t, sizes, grad, type), "a saved tensor is another in the backward pass (replaced, or unpacked by a saved-tensor hook) than the forward pass saved");
   return dense(t);
 }
 
@@ -146,7 +146,8 @@ struct Linear : public Function<Linear> {
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
     const Tensor dy = dense(grads[0]), weight = kept_weight(ctx);
-    const int64_t N = weight.size(0), K = weight.size(1), M = dy.numel() / N;
+    // the gradient's shape is the output's; a weight whose data was replaced since is refused with the saved one
+    const int64_t N = dy.size(-1), K = weight.size(-1), M = dy.numel() / N;
     auto sizes = dy.sizes().vec();
     sizes.back() = K;
     const Tensor x = operand(saved[0], sizes, dy), w = operand(saved[1], {N, K}, dy);
