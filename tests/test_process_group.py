@@ -3,9 +3,12 @@ collective of the torchft contract against each backend, as the reference's
 process_group_test.py does."""
 
 import gc
+import os
+import signal
+import time
 from concurrent.futures import ThreadPoolExecutor
 from datetime import timedelta
-from unittest.mock import MagicMock, create_autospec
+from unittest.mock import MagicMock, create_autospec, patch
 
 import pytest
 import torch
@@ -155,6 +158,25 @@ def test_baby_gloo_conformance_and_reconfigure():
         assert pg.getBackendName() == "torchft-baby-gloo"
     finally:
         pg.shutdown()
+
+
+def test_baby_gloo_child_drops_its_works_before_it_is_killed():
+    """shutdown() lets the child give back what it was sent; a child that does not answer is killed after a moment."""
+    store = make_store()
+    pg = ProcessGroupBabyGloo(timeout=timedelta(seconds=20))
+    pg.configure(f"127.0.0.1:{store.port}/end", 0, 1)
+    work = pg.allreduce([torch.ones(4)], ReduceOp.SUM)
+    work.wait()
+    replies, taken = pg._reply_q, []
+    with patch("torchft_b200.process_group._take_reply", side_effect=lambda q, t: taken.append((q, q.get(timeout=20)))):
+        pg.shutdown()
+    assert taken == [(replies, ("stopped", None))]
+    pg.configure(f"127.0.0.1:{store.port}/end2", 0, 1)
+    child = pg._p
+    os.kill(child.pid, signal.SIGSTOP)
+    begin = time.monotonic()
+    pg.shutdown()
+    assert not child.is_alive() and time.monotonic() - begin < 15
 
 
 def test_baby_gloo_start_timeout():

@@ -8,6 +8,9 @@ cases, and a rank that leaves while bound to an NVLink multicast object disturbs
 
 import gc
 import os
+import subprocess
+import sys
+import tempfile
 from concurrent.futures import ThreadPoolExecutor
 from datetime import timedelta
 
@@ -18,6 +21,7 @@ from torch.distributed import ReduceOp, TCPStore
 
 os.environ.setdefault("NCCL_NVLS_ENABLE", "0")
 
+from conftest import ROOT  # noqa: E402
 from test_process_group import check_collectives  # noqa: E402 - the conformance helper of the CPU tests
 
 pytestmark = pytest.mark.gpu
@@ -61,6 +65,44 @@ def test_baby_nccl_api_surface_and_work_bookkeeping():
         assert pg.num_active_work() == 0  # ... so the child dropped its side too
     finally:
         pg.shutdown()
+
+
+def test_a_program_with_a_baby_group_exits_cleanly():
+    """The child gives back the tensors it was sent, also when it is replaced, and at shutdown those of works still held, and the
+    sender takes them off torch's list of shared memory.  What stays there is cleared while the process exits, with a warning or
+    a segmentation fault at times."""
+    code = """
+import gc, torch
+from datetime import timedelta
+from torch.distributed import ReduceOp, TCPStore
+from torchft_b200.process_group import ProcessGroupBabyNCCL
+
+def main():
+    store = TCPStore(host_name="127.0.0.1", port=0, is_master=True, wait_for_workers=False)
+    pg = ProcessGroupBabyNCCL(timeout=timedelta(seconds=60))
+    for attempt in range(2):
+        pg.configure(f"127.0.0.1:{store.port}/exit{attempt}", 0, 1)
+        work = pg.allreduce([torch.ones(1 << 20, device="cuda")], ReduceOp.SUM)
+        work.wait()
+        torch.cuda.synchronize()
+        if attempt == 0:
+            del work
+            gc.collect()
+            assert pg.num_active_work() == 0
+    pg.shutdown()
+    assert torch.cuda.memory_allocated() == 0, torch.cuda.memory_allocated()
+
+if __name__ == "__main__":
+    main()
+"""
+    with tempfile.TemporaryDirectory() as folder:
+        script = os.path.join(folder, "program.py")
+        with open(script, "w") as f:
+            f.write(code)
+        env = dict(os.environ, PYTHONPATH=os.pathsep.join(filter(None, (str(ROOT), os.environ.get("PYTHONPATH")))))
+        done = subprocess.run([sys.executable, script], env=env, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr
+    assert "shared CUDA tensors released" not in done.stderr
 
 
 def test_baby_nccl_two_gpus():
